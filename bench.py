@@ -307,7 +307,7 @@ def run_lux(a):
         "config": {"workload": DESC,
                    "parallelism": f"replicas x{world}", "l2": l2_note(),
                    "stages_ms": {"cost": cost_ms, "sgm_2_passes": sgm_ms, "wta": wta_ms},
-                   "sgm_kernel": {0: "exact-replay", 1: "fused-wavefront", 2: "path-group-chains", 3: "lean-wavefront"}.get(
+                   "sgm_kernel": {0: "exact-replay", 1: "fused-wavefront", 2: "path-group-chains", 3: "lean-wavefront", 4: "lines"}.get(
                        inf_v[0][3] if inf_v else -1)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk.get("hbm_gbs"), "unit": "GB/s",
                      "frac": achieved / pk.get("hbm_gbs"), "traffic": TRAFFIC_PER_DE_LAYER * de,

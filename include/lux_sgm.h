@@ -161,7 +161,7 @@ typedef struct {
   float gpu_ms_sgm;      /* device time of the two aggregation passes */
   float gpu_ms_wta;      /* device time of the winner-take-all */
   int32_t sgm_kernel;    /* 0 = the exact traversal replay, 1 = fast, four paths fused, 2 = fast, path groups as chains,
-                            3 = fast, four paths fused, lean wavefront */
+                            3 = fast, four paths fused, lean wavefront, 4 = fast, every path along its own lines */
   int32_t cost_kernel;   /* 0 = per-pixel warps (any layer), 1 = per-row warps (uniform layer), 2 = per-row warps of an axis-aligned
                             pair, 3 = the same with block columns shared between neighbouring pixels (grey, scale 1) */
   int32_t tuned;         /* the fast form the autotuner chose on this solve (it timed every form), 0 when it did not run */

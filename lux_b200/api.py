@@ -748,7 +748,7 @@ class ServedResult:
     run_ms: float
 
 
-SGM_FORM_NAMES = {1: "fused", 2: "split", 3: "wave"}
+SGM_FORM_NAMES = {1: "fused", 2: "split", 3: "wave", 4: "lines"}
 
 
 def tuned_form(w, h, n_planes, tile) -> int:

@@ -177,6 +177,12 @@ int run_sgm_split(const LayerGeom& g, int xsw, uint16_t p1, float p2scale, const
 size_t wave_scratch_bytes(int W, int H, int n);
 int run_sgm_wave(const LayerGeom& g, int xsw, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg,
                  uint16_t* agg_pass1, float* depth, int keep_agg, void* scratch, size_t scratch_bytes, int* err, cudaStream_t s);
+// sgm_lines.cu: the same aggregation one path at a time along independent lines (n <= 256; pass +1's aggregates never exist
+// by themselves, so it cannot keep them)
+bool lines_supported(int W, int n);
+size_t lines_scratch_bytes(int W, int H, int n);
+int run_sgm_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg, float* depth,
+                  int keep_agg, void* scratch, size_t scratch_bytes, cudaStream_t s);
 int run_sgm_uniform(const LayerGeom& g, int xsw, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg,
                     uint16_t* agg_pass1, float* depth, int keep_agg, void* scratch, size_t scratch_bytes, int* err,
                     cudaStream_t s);

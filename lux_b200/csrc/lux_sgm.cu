@@ -48,15 +48,19 @@ struct DevBuf {
 // that shape.
 namespace {
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, int> g_tuned;
-int tuned_form(int W, int H, int n, int T) {
+struct TunedForm {
+  int form = 0;
+  bool set_by_caller = false;  // lux_sgm_set_tuned_form: also followed where the lines form would run
+};
+std::map<std::tuple<int, int, int, int>, TunedForm> g_tuned;
+TunedForm tuned_form(int W, int H, int n, int T) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tuned.find(std::make_tuple(W, H, n, T));
-  return it == g_tuned.end() ? 0 : it->second;
+  return it == g_tuned.end() ? TunedForm{} : it->second;
 }
-void set_tuned_form(int W, int H, int n, int T, int form) {
+void set_tuned_form(int W, int H, int n, int T, int form, bool by_caller) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  if (form) g_tuned[std::make_tuple(W, H, n, T)] = form;
+  if (form) g_tuned[std::make_tuple(W, H, n, T)] = TunedForm{form, by_caller};
   else g_tuned.erase(std::make_tuple(W, H, n, T));
 }
 }  // namespace
@@ -270,6 +274,8 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     std::vector<DevBuf>* t;
     ~TmpGuard() { dev_free_all(c, *t); }
   } guard{ctx, &tmp};
+  std::vector<DevBuf> phases;  // the phase images: the aggregation's scratch may reuse their memory once the cost has run
+  TmpGuard phase_guard{ctx, &phases};
   bool uniform = prev == nullptr;
   if (uniform) {  // DenseStereoSgm.cs:43-46
     launch_uniform_ranges(L->start, L->count, L->cap, L->off, (int)npx, L->n, s);
@@ -366,12 +372,13 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
   const size_t phase_words = cost_all_grey(ca) ? 8 : 4;  // per pixel: four phases of {u16 pairs} (grey) or RGBA words
   for (int k = 0; k < ca.n_others; k++) {  // the half-pixel phase images of the other cameras
     uint32_t* ph = nullptr;
-    if ((rc = alloc_t(ctx, tmp, phase_words * ca.ow[k] * ca.oh[k], &ph))) return rc;
+    if ((rc = alloc_t(ctx, phases, phase_words * ca.ow[k] * ca.oh[k], &ph))) return rc;
     ca.phase[k] = ph;
   }
   CK(cudaEventRecord(ctx->ev[0], s));
   launch_phases(ca, s);
   L->cost_kernel = launch_cost(ca, g, zt, L->raw, ctx->d_err, s);
+  dev_free_all(ctx, phases);
   // aggregation: two passes over the sheared tiles, then WTA
   CK(cudaEventRecord(ctx->ev[1], s));
   const int xsw = 0;  // LUX_SGM_XSW unset: the reference default (DenseStereoSgm.cs:31)
@@ -382,15 +389,23 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     int form = forced;
     bool tune = false;
     if (!forced) {
-      form = tuned_form(W, H, L->n, p.tile);
-      tune = form == 0 && ctx->autotune;
-      if (form == 0) form = (size_t)W * H >= 2000000 ? 2 : 1;  // untuned: the path-group chains from about 2 MP
+      const TunedForm t = tuned_form(W, H, L->n, p.tile);
+      // The lines form is faster than the other three at every size (4160x3120 D=256: 15.4 against 17.6 ms; 1040x780
+      // D=64: 0.66 against 4.5 ms; 520x390 D=32: 0.29 against 2.4 ms) but never holds pass +1's aggregates alone and waits on nothing (debug_stall).
+      if (!(flags & LUX_LAYER_KEEP_PASS1) && !t.set_by_caller && ctx->stall_block < 0 && lines_supported(W, L->n)) {
+        form = 4;
+      } else {
+        form = t.form;
+        tune = form == 0 && ctx->autotune;
+        if (form == 0) form = (size_t)W * H >= 2000000 ? 2 : 1;  // untuned: the path-group chains from about 2 MP
+      }
     }
     const int keep = (flags & LUX_LAYER_KEEP_AGG) ? 1 : 0;
     auto scratch_of = [&](int f) {
-      return f == 2 ? split_scratch_bytes(W, H, L->n) : f == 3 ? wave_scratch_bytes(W, H, L->n) : uniform_scratch_bytes(W, H, L->n, p.tile);
+      return f == 4 ? lines_scratch_bytes(W, H, L->n) : f == 2 ? split_scratch_bytes(W, H, L->n) : f == 3 ? wave_scratch_bytes(W, H, L->n) : uniform_scratch_bytes(W, H, L->n, p.tile);
     };
     auto run_form = [&](int f, void* scr, size_t sb) {
+      if (f == 4) return run_sgm_lines(g, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->depth, keep, scr, sb, s);
       if (f == 2) return run_sgm_split(g, xsw, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->agg_pass1, L->depth, keep, scr, sb, ctx->d_err, s);
       if (f == 3) return run_sgm_wave(g, xsw, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->agg_pass1, L->depth, keep, scr, sb, ctx->d_err, s);
       return run_sgm_uniform(g, xsw, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->agg_pass1, L->depth, keep, scr, sb, ctx->d_err, s);
@@ -424,7 +439,7 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
           best_ms = ms;
         }
       }
-      set_tuned_form(W, H, L->n, p.tile, best);
+      set_tuned_form(W, H, L->n, p.tile, best, false);
       L->sgm_kernel = kForms[2];  // the last run's results are in place
       L->agg_final = keep != 0;
       L->ms_sgm = best_ms;
@@ -569,11 +584,11 @@ int lux_sgm_set_autotune(lux_sgm_ctx* ctx, int32_t on) {
   return LUX_OK;
 }
 
-int32_t lux_sgm_tuned_form(int32_t w, int32_t h, int32_t n_planes, int32_t tile) { return tuned_form(w, h, n_planes, tile); }
+int32_t lux_sgm_tuned_form(int32_t w, int32_t h, int32_t n_planes, int32_t tile) { return tuned_form(w, h, n_planes, tile).form; }
 
 int lux_sgm_set_tuned_form(int32_t w, int32_t h, int32_t n_planes, int32_t tile, int32_t form) {
   if (w <= 0 || h <= 0 || n_planes <= 0 || tile <= 0 || form < 0 || form > 3) return LUX_ERR_ARG;
-  set_tuned_form(w, h, n_planes, tile, form);
+  set_tuned_form(w, h, n_planes, tile, form, true);
   return LUX_OK;
 }
 
