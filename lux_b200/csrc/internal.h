@@ -183,6 +183,13 @@ bool lines_supported(int W, int n);
 size_t lines_scratch_bytes(int W, int H, int n);
 int run_sgm_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg, float* depth,
                   int keep_agg, void* scratch, size_t scratch_bytes, cudaStream_t s);
+// sgm_ragged.cu: the same for ragged layers and uniform ones past 256 planes. *flag (device) becomes 1 where the layer's ranges
+// meet the ends of the reference's line buffer in a way that only the exact replay follows.
+void launch_ragged_check(const LayerGeom& g, int* flag, cudaStream_t s);
+bool ragged_lines_supported(int W, int H, int tile, uint16_t p1, float p2scale, int max_hi, uint64_t volume);
+size_t ragged_lines_scratch_bytes(int W, int H, int max_hi);
+int run_ragged_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg, void* scratch,
+                     size_t scratch_bytes, cudaStream_t s);
 int run_sgm_uniform(const LayerGeom& g, int xsw, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg,
                     uint16_t* agg_pass1, float* depth, int keep_agg, void* scratch, size_t scratch_bytes, int* err,
                     cudaStream_t s);
