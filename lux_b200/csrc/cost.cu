@@ -643,6 +643,373 @@ __global__ void __launch_bounds__(256, P > 2 ? 3 : 4)
   }
 }
 
+// ---------------- an axis-aligned grey pair of one focal length at scale 1 ----------------
+//
+// Every target then lies a whole number of half pixels from its pixel, the same number along a row and along a column for
+// most planes; rounding tips positions of a plane whose shift falls near the middle of two half pixels to one or the other.
+// k_unit_planes evaluates the reference's projection for every column and every row of every plane and records, per plane,
+// the shift in half pixels and the interval of in-rect columns and rows, or that two shifts occur, or more.
+//
+// k_cost_unit then works on bytes, four neighbouring pixels a word: |t - r| by the byte-wise absolute difference, capped at
+// 2, summed over the three rows, then over three columns (the neighbouring bytes; from the lanes beside at a word's ends):
+// at most 18, no carry. The normalised cost is one multiply of two sums a word (cost_unit_norm). A warp (a block by itself,
+// so that the plane's scalars and the row addresses stay on the uniform datapath) takes a run of 120
+// pixels (lanes 0 and 31 only supply their columns) of kUnitRows rows, sharing the capped differences of the rows between
+// them, and 32 planes at a time through shared memory, so that a pixel's costs go out in 32-byte pieces. A plane of two
+// shifts makes the costs of both and selects by each pixel's own target; plane 0 (clamped into the rect) and planes of more
+// gather each block by itself. The byte phase images come in four copies, each a byte further on, so that every word load
+// is aligned. Bound by the ALU pipe (64 operations a plane, row and warp: 128 pixels): 4160x3120 D=256 takes 2.2 ms
+// (k_cost_axis_v 7.7), 2080x1560 D=256 0.61 (1.97), 1040x780 D=64 0.080 (0.163). Three rows a warp: 2.1, 0.65, 0.089.
+constexpr int kUnitRows = 2, kUnitRun = 120, kUnitPad = 256;
+__host__ __device__ constexpr int unit_pitch(int w) { return (w + 2 * kUnitPad + 127) & ~127; }
+struct UnitPlane {
+  int dx, xa, xb;  // columns xa..xb-1 are in the rect, 2·column + dx half pixels (or dx + 1 where two_x)
+  int dy, ya, yb;  // rows likewise
+  int two_x, two_y;
+  int whole;       // the intervals and shifts say it all
+  int other;       // more shifts than two, or gaps in an interval
+  int pad[2];
+};
+
+size_t cost_unit_phase_bytes(int w, int h, int n_planes) {
+  return (size_t)16 * h * unit_pitch(w) + (size_t)n_planes * sizeof(UnitPlane);
+}
+LUX_DEV const UnitPlane* unit_planes(const CostArgs& a) {
+  return reinterpret_cast<const UnitPlane*>(reinterpret_cast<const uint8_t*>(a.phase[0]) + (size_t)16 * a.oh[0] * unit_pitch(a.ow[0]));
+}
+
+// Byte phase images: out[h][k][y][i] = phase h at column i + k - kUnitPad (clamped to the image). A thread makes four bytes of
+// the four copies of every phase.
+__global__ void k_phase_bytes(const uint8_t* __restrict__ img, int iw, int ih, uint8_t* __restrict__ out) {
+  const int pitch = unit_pitch(iw), i4 = (blockIdx.x * blockDim.x + threadIdx.x) * 4, y = blockIdx.y;
+  if (i4 >= pitch) return;
+  const int y1 = min(y + 1, ih - 1);
+  int r0[8], r1[8];  // columns i4 - kUnitPad .. + 7 of rows y and y + 1
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const int x = min(max(i4 + c - kUnitPad, 0), iw - 1);
+    r0[c] = __ldg(img + ((size_t)y * iw + x) * 4);
+    r1[c] = __ldg(img + ((size_t)y1 * iw + x) * 4);
+  }
+#pragma unroll
+  for (int h = 0; h < 4; h++) {
+    int v[8];
+#pragma unroll
+    for (int c = 0; c < 7; c++) {
+      const int a = h & 2 ? avg_u8(r0[c], r1[c]) : r0[c], b = h & 2 ? avg_u8(r0[c + 1], r1[c + 1]) : r0[c + 1];
+      v[c] = h & 1 ? avg_u8(a, b) : a;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      *reinterpret_cast<uint32_t*>(out + ((size_t)(h * 4 + k) * ih + y) * pitch + i4) =
+          (uint32_t)v[k] | (uint32_t)v[k + 1] << 8 | (uint32_t)v[k + 2] << 16 | (uint32_t)v[k + 3] << 24;
+  }
+}
+
+// The half-pixel target position of coordinate v of a plane (k_cost_axis's projection): w the flow-matrix factor of the axis.
+LUX_DEV int unit_target(float v, float z, float zt, float inv, float w) {
+  const float f = __fadd_rn(__fmul_rn(__fadd_rn(zt, __fmul_rn(__fmul_rn(v, z), w)), inv), 0.25f);
+  return f2i(__fadd_rn(f, f));
+}
+__global__ void __launch_bounds__(256) k_unit_planes(const CostArgs a, const LayerGeom g, const float4* __restrict__ zt, UnitPlane* __restrict__ out) {
+  __shared__ int s_dlo[2], s_dhi[2], s_lo[2], s_hi[2], s_cnt[2];
+  const int p = blockIdx.x, t = threadIdx.x;
+  const float z = g.planes[p];
+  const float4 zk = zt[p];
+  if (t < 2) {
+    s_dlo[t] = s_lo[t] = INT_MAX;
+    s_dhi[t] = INT_MIN;
+    s_hi[t] = s_cnt[t] = 0;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int ax = 0; ax < 2; ax++) {
+    const int n = ax ? g.H : g.W, lim = (ax ? a.oh[0] : a.ow[0]) - 2;
+    int lo = INT_MAX, hi = 0, cnt = 0, dlo = INT_MAX, dhi = INT_MIN;
+    for (int v = t; v < n; v += 256) {
+      const int q = unit_target((float)v, z, ax ? zk.y : zk.x, zk.w, ax ? a.warp[0][5] : a.warp[0][0]), iq = q >> 1;
+      if (iq >= 1 && iq < lim) {
+        lo = min(lo, v);
+        hi = v + 1;
+        cnt++;
+        dlo = min(dlo, q - 2 * v);
+        dhi = max(dhi, q - 2 * v);
+      }
+    }
+    if (cnt) {
+      atomicMin(&s_lo[ax], lo);
+      atomicMax(&s_hi[ax], hi);
+      atomicAdd(&s_cnt[ax], cnt);
+      atomicMin(&s_dlo[ax], dlo);
+      atomicMax(&s_dhi[ax], dhi);
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    UnitPlane u;
+    const bool none = s_cnt[0] == 0 || s_cnt[1] == 0;  // nothing in the rect
+    u.dx = none ? 0 : s_dlo[0];
+    u.xa = none ? 0 : s_lo[0];
+    u.xb = none ? 0 : s_hi[0];
+    u.dy = none ? 0 : s_dlo[1];
+    u.ya = none ? 0 : s_lo[1];
+    u.yb = none ? 0 : s_hi[1];
+    u.two_x = !none && s_dhi[0] == u.dx + 1;
+    u.two_y = !none && s_dhi[1] == u.dy + 1;
+    u.other = !none && (s_dhi[0] > u.dx + 1 || s_dhi[1] > u.dy + 1 || s_cnt[0] != u.xb - u.xa || s_cnt[1] != u.yb - u.ya);
+    u.whole = !u.two_x && !u.two_y && !u.other;
+    u.pad[0] = u.pad[1] = 0;
+    out[p] = u;
+  }
+}
+
+uint32_t cost_unit_norm(float norm) {
+  uint8_t tab[19];
+  for (int s = 0; s < 19; s++) {
+    volatile float v = (float)((uint32_t)(s * 12240 + 16) >> 5) * norm;
+    tab[s] = (uint8_t)(int)v;
+  }
+  for (uint32_t m = 0; m <= 65535 / 18; m++) {
+    bool ok = true;
+    for (uint32_t s = 0; s < 19 && ok; s++) ok = (s * m) >> 8 == tab[s];
+    if (ok) return m;
+  }
+  return 0;
+}
+
+// min(|t - r|, 2) of four bytes: bit 7 of `big` says a difference of 2 or more.
+LUX_DEV uint32_t capped_diff4(uint32_t t, uint32_t r) {
+  const uint32_t v = __vabsdiffu4(t, r);
+  const uint32_t big = ((v & 0x7e7e7e7eu) + 0x7e7e7e7eu) | v;
+  const uint32_t two = (big >> 6) & 0x02020202u;
+  return two | (v & ~(two >> 1) & 0x01010101u);
+}
+
+// One pixel's block at a plane by itself: its raw sum S0, or -1 where the target leaves the rect.
+LUX_DEV int unit_gather(const CostArgs& a, const LayerGeom& g, const float4* __restrict__ zt, const uint8_t* bytes, int pitch, int x, int y, int p) {
+  const int iw = a.ow[0], ih = a.oh[0], x1 = iw - 2, y1 = ih - 2;
+  const float z = __ldg(g.planes + p), xf = (float)x, yf = (float)y;
+  const float4 zk = __ldg(zt + p);
+  int tx, ty;
+  if (p == 0) {  // the general projection, clamped into the rect (:263-269)
+    const float* Wm = a.warp[0];
+    const float xz = __fmul_rn(xf, z), yz = __fmul_rn(yf, z);
+    const float px = __fadd_rn(__fadd_rn(zk.x, __fmul_rn(xz, Wm[0])), __fmul_rn(yz, Wm[4]));
+    const float py = __fadd_rn(__fadd_rn(zk.y, __fmul_rn(xz, Wm[1])), __fmul_rn(yz, Wm[5]));
+    const float pz = __fadd_rn(__fadd_rn(zk.z, __fmul_rn(xz, Wm[2])), __fmul_rn(yz, Wm[6]));
+    const float inv = __frcp_rn(pz);
+    const float fx = cs_minf(cs_maxf(__fadd_rn(__fmul_rn(px, inv), 0.25f), 1.0f), (float)(x1 - 1));
+    const float fy = cs_minf(cs_maxf(__fadd_rn(__fmul_rn(py, inv), 0.25f), 1.0f), (float)(y1 - 1));
+    tx = f2i(__fadd_rn(fx, fx));
+    ty = f2i(__fadd_rn(fy, fy));
+  } else {
+    tx = unit_target(xf, z, zk.x, zk.w, a.warp[0][0]);
+    ty = unit_target(yf, z, zk.y, zk.w, a.warp[0][5]);
+  }
+  const int ix = tx >> 1, iy = ty >> 1;
+  if (ix < 1 || ix >= x1 || iy < 1 || iy >= y1) return -1;
+  const uint8_t* q = bytes + ((size_t)(((ty & 1) << 1) | (tx & 1)) * 4 * ih + (iy - 1)) * pitch + kUnitPad + ix - 1;
+  int s = 0;
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const uint8_t* rr = a.ref + (size_t)min(max(y + r - 1, 0), a.rh - 1) * a.rw * 4;
+#pragma unroll
+    for (int c = 0; c < 3; c++) s += min(abs((int)__ldg(q + (size_t)r * pitch + c) - (int)__ldg(rr + (size_t)min(max(x + c - 1, 0), a.rw - 1) * 4)), 2);
+  }
+  return s;
+}
+
+__global__ void __launch_bounds__(32) k_cost_unit(const CostArgs a, const LayerGeom g, const float4* __restrict__ zt, uint8_t* __restrict__ raw, int* err) {
+  constexpr int R = kUnitRows;
+  __shared__ uint32_t s_out[R][128][8];  // 32 planes of a pixel, words swizzled by the pixel
+  const int lane = threadIdx.x, runs = (g.W + kUnitRun - 1) / kUnitRun, tile = blockIdx.x;
+  const int n = g.n_planes, ih = a.oh[0], pitch = unit_pitch(a.ow[0]);
+  const uint8_t* bytes = reinterpret_cast<const uint8_t*>(a.phase[0]);
+  const UnitPlane* up = unit_planes(a);
+  const int y0 = tile / runs * R, X0 = (tile % runs) * kUnitRun - 4, x0 = X0 + 4 * lane;  // columns X0..X0+127, x0: this lane's
+  const bool stores = lane >= 1 && lane <= 30;
+  uint32_t ref[R + 2], keep[R], last[R];
+#pragma unroll
+  for (int r = 0; r < R + 2; r++) {  // rows y0-1..y0+R and the columns, clamped as the reference clamps its block
+    const uint8_t* row = a.ref + (size_t)min(max(y0 + r - 1, 0), a.rh - 1) * a.rw * 4;
+    uint32_t w = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) w |= (uint32_t)__ldg(row + (size_t)min(max(x0 + j, 0), a.rw - 1) * 4) << (8 * j);
+    ref[r] = w;
+  }
+#pragma unroll
+  for (int i = 0; i < R; i++) {  // skipped pixels' costs are 0 (DenseStereoSgm.cs:242)
+    keep[i] = 0;
+    last[i] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (stores && x0 + j < g.W && y0 + i < g.H && g.skip[(size_t)(y0 + i) * g.W + x0 + j] == 0) keep[i] |= 0xffu << (8 * j);
+  }
+  const uint32_t mul = a.norm_mul;
+  auto gather = [&](int p) {  // the blocks one by one
+#pragma unroll
+    for (int i = 0; i < R; i++)
+#pragma unroll 1
+      for (int j = 0; j < 4; j++) {
+        if (!((keep[i] >> (8 * j)) & 1)) continue;
+        const int s = unit_gather(a, g, zt, bytes, pitch, x0 + j, y0 + i, p);
+        if (s >= 0) last[i] = (last[i] & ~(0xffu << (8 * j))) | (((uint32_t)s * mul) >> 8) << (8 * j);
+        else if (p == 0) atomicCAS(err, 0, 7);  // the scalar fallback of the reference would read out of the image
+      }
+  };
+  // The costs of a plane whose block rows' capped differences are d[] (four pixels a word).
+  auto sums = [&](const uint32_t (&d)[R + 2], uint32_t (&c)[R]) {
+#pragma unroll
+    for (int i = 0; i < R; i++) {
+      const uint32_t v = d[i] + d[i + 1] + d[i + 2];
+      const uint32_t left = __shfl_up_sync(0xffffffffu, v, 1), right = __shfl_down_sync(0xffffffffu, v, 1);
+      const uint32_t t = v + __byte_perm(left, v, 0x6543) + __byte_perm(v, right, 0x4321);
+      c[i] = __byte_perm((t & 0x00ff00ffu) * mul, ((t >> 8) & 0x00ff00ffu) * mul, 0x7351);
+    }
+  };
+  auto plane = [&](int p) {  // makes last[] the costs of plane p
+    const UnitPlane u = up[p];
+    if (p == 0 || u.other) {
+      gather(p);
+      return;
+    }
+    if (u.xa >= X0 + 128 || u.xb <= X0 || u.ya >= y0 + R || u.yb <= y0) return;  // nothing in the rect: the last cost stays (:273-274)
+    const float z = __ldg(g.planes + p);
+    const float4 zk = __ldg(zt + p);
+    uint32_t made[R];  // the costs made so far, each pixel's at its own shift
+#pragma unroll
+    for (int i = 0; i < R; i++) made[i] = last[i];
+#pragma unroll 1
+    for (int v = 0; v < 4; v++) {
+      const int dx = u.dx + (v & 1), dy = u.dy + (v >> 1);
+      if (((v & 1) && !u.two_x) || ((v >> 1) && !u.two_y)) continue;
+      const int o = x0 + (dx >> 1) + kUnitPad;  // its low two bits are the warp's
+      const uint8_t* base = bytes + (size_t)((((dy & 1) << 1) | (dx & 1)) * 4 + (o & 3)) * ih * pitch + (o & ~3);
+      uint32_t d[R + 2], c[R];
+#pragma unroll
+      for (int r = 0; r < R + 2; r++) {
+        const int row = min(max(y0 + r - 1 + (dy >> 1), 0), ih - 1);
+        d[r] = capped_diff4(__ldg(reinterpret_cast<const uint32_t*>(base + (size_t)row * pitch)), ref[r]);
+      }
+      sums(d, c);
+      uint32_t mask = 0;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const bool mine = !u.two_x || unit_target((float)(x0 + j), z, zk.x, zk.w, a.warp[0][0]) - 2 * (x0 + j) == dx;
+        if (mine && x0 + j >= u.xa && x0 + j < u.xb) mask |= 0xffu << (8 * j);
+      }
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        const int y = y0 + i;
+        const bool mine = !u.two_y || unit_target((float)y, z, zk.y, zk.w, a.warp[0][5]) - 2 * y == dy;
+        if (mine && y >= u.ya && y < u.yb) made[i] = (c[i] & mask) | (made[i] & ~mask);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R; i++) last[i] = made[i];
+  };
+  const bool full_run = X0 + 124 <= g.W;
+#pragma unroll 1
+  for (int p0 = 0; p0 < n; p0 += 32) {
+    const int m = min(32, n - p0);
+    // lane i: plane p0 + i over this tile: all in the rect with one shift (plain), the same but for columns outside xa..xb-1
+    // (partly), nothing in the rect (none), or any other (by itself); and where the tile's first block row starts
+    uint32_t off = 0;
+    int xa = 0, xb = 0;
+    bool plain = false, partly = false, none = false;
+    if (lane < m && p0 + lane > 0) {
+      const UnitPlane u = up[p0 + lane];
+      xa = u.xa;
+      xb = u.xb;
+      none = u.whole && (u.xa >= X0 + 128 || u.xb <= X0 || u.ya >= y0 + R || u.yb <= y0);
+      partly = u.whole && !none && u.ya <= y0 && u.yb >= y0 + R;
+      plain = partly && u.xa <= X0 && u.xb >= X0 + 128;
+      const int o = X0 + (u.dx >> 1) + kUnitPad, h = ((u.dy & 1) << 1) | (u.dx & 1);
+      if (partly) off = ((uint32_t)(h * 4 + (o & 3)) * ih + (uint32_t)(y0 - 1 + (u.dy >> 1))) * (uint32_t)pitch + (uint32_t)(o & ~3);
+    }
+    const uint32_t plain_planes = __ballot_sync(0xffffffffu, plain), none_planes = __ballot_sync(0xffffffffu, none);
+    const uint32_t masked_planes = __ballot_sync(0xffffffffu, partly) | none_planes;
+#pragma unroll 1
+    for (int q = 0; q < m; q += 4) {
+      uint32_t c[4][R];  // four planes of four pixels
+      if (((none_planes >> q) & 15u) == 15u) {  // the last cost stays (:273-274)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+          for (int i = 0; i < R; i++) c[k][i] = last[i];
+      } else if (((masked_planes >> q) & 15u) == 15u) {
+        uint32_t t[4][R + 2];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {  // (planes with nothing in the rect read some words and keep none)
+          const uint8_t* b = bytes + __shfl_sync(0xffffffffu, off, q + k) + 4 * lane;
+#pragma unroll
+          for (int r = 0; r < R + 2; r++, b += pitch) t[k][r] = __ldg(reinterpret_cast<const uint32_t*>(b));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+#pragma unroll
+          for (int r = 0; r < R + 2; r++) t[k][r] = capped_diff4(t[k][r], ref[r]);
+          sums(t[k], c[k]);
+        }
+        if (((plain_planes >> q) & 15u) != 15u) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            int lo = min(max(__shfl_sync(0xffffffffu, xa, q + k) - x0, 0), 4), hi = min(max(__shfl_sync(0xffffffffu, xb, q + k) - x0, 0), 4);
+            if ((none_planes >> (q + k)) & 1) lo = 4;
+            const uint32_t mask = (lo < 4 ? 0xffffffffu << (8 * lo) : 0u) & (hi < 4 ? (1u << (8 * hi)) - 1u : 0xffffffffu);
+#pragma unroll
+            for (int i = 0; i < R; i++) c[k][i] = (c[k][i] & mask) | ((k ? c[k > 0 ? k - 1 : 0][i] : last[i]) & ~mask);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < R; i++) last[i] = c[3][i];
+      } else {
+#pragma unroll 1
+        for (int k = 0; k < 4; k++) {
+          plane(p0 + q + k);
+#pragma unroll
+          for (int i = 0; i < R; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+              reinterpret_cast<uint8_t*>(&s_out[i][j * 32 + lane][(q >> 2) ^ ((lane >> 2) & 7)])[k] = (uint8_t)((last[i] & keep[i]) >> (8 * j));
+        }
+        continue;
+      }
+#pragma unroll
+      for (int i = 0; i < R; i++) {  // transposed: four planes of a pixel a word
+        const uint32_t a0 = __byte_perm(c[0][i] & keep[i], c[1][i] & keep[i], 0x5140), a1 = __byte_perm(c[2][i] & keep[i], c[3][i] & keep[i], 0x5140),
+                       b0 = __byte_perm(c[0][i] & keep[i], c[1][i] & keep[i], 0x7362), b1 = __byte_perm(c[2][i] & keep[i], c[3][i] & keep[i], 0x7362);
+        uint32_t* o = &s_out[i][lane][(q >> 2) ^ ((lane >> 2) & 7)];
+        o[0] = __byte_perm(a0, a1, 0x5410);
+        o[32 * 8] = __byte_perm(a0, a1, 0x7632);
+        o[64 * 8] = __byte_perm(b0, b1, 0x5410);
+        o[96 * 8] = __byte_perm(b0, b1, 0x7632);
+      }
+    }
+    __syncwarp();
+    // a pixel's planes by eight lanes (32 bytes), four pixels at a time: word l, byte j of the run is pixel X0 + 4l + j
+    const int w = lane & 7, sub = lane >> 3;
+    if (w * 4 < m) {
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        if (y0 + i >= g.H) break;
+#pragma unroll 1
+        for (int j = 0; j < 4; j++) {
+          const int xj = X0 + 4 * sub + j;
+          uint8_t* o = raw + ((long long)(y0 + i) * g.W + xj) * n + p0 + w * 4;
+          const uint32_t* src = &s_out[i][j * 32 + sub][0];
+#pragma unroll
+          for (int k = 0; k < 8; k++, o += 16 * n) {
+            if ((k > 0 || sub > 0) && (k < 7 || sub < 3) && (full_run || xj + 16 * k < g.W))
+              *reinterpret_cast<uint32_t*>(o) = src[k * 32 + (w ^ k)];
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
 bool cost_all_grey(const CostArgs& a) {
   for (int k = 0; k < a.n_others; k++)
     if (!(a.wq[k][0] == 12240 && a.wq[k][1] == 0 && a.wq[k][2] == 0 && a.wq[k][3] == 0)) return false;
@@ -654,7 +1021,9 @@ void launch_phases(const CostArgs& a, cudaStream_t s) {
   for (int k = 0; k < a.n_others; k++) {
     dim3 grid((a.ow[k] + 127) / 128, a.oh[k]);
     uint32_t* out = const_cast<uint32_t*>(a.phase[k]);
-    if (a.vcols) k_phase_grey_v<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint2*>(out));
+    if (a.unit)
+      k_phase_bytes<<<dim3((unit_pitch(a.ow[k]) / 4 + 127) / 128, a.oh[k]), 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint8_t*>(out));
+    else if (a.vcols) k_phase_grey_v<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint2*>(out));
     else if (grey) k_phase_grey<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint2*>(out));
     else k_phase_colour<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], out);
     count_launches(1);
@@ -687,7 +1056,14 @@ int launch_cost(const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t
     const int tiles = ((g.W + 31) / 32) * g.H;
     int blocks = (tiles + 7) / 8;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    if (a.vcols) {
+    if (a.unit) {
+      uint8_t* ph = reinterpret_cast<uint8_t*>(const_cast<uint32_t*>(a.phase[0]));
+      k_unit_planes<<<g.n_planes, 256, 0, s>>>(a, g, zt, reinterpret_cast<UnitPlane*>(ph + (size_t)16 * a.oh[0] * unit_pitch(a.ow[0])));
+      count_launches(1);
+      const int tiles_u = ((g.W + kUnitRun - 1) / kUnitRun) * ((g.H + kUnitRows - 1) / kUnitRows);
+      k_cost_unit<<<tiles_u, 32, 0, s>>>(a, g, zt, raw, err);
+      kind = 3;
+    } else if (a.vcols) {
       const int vruns = ((g.W + kAxRun - 1) / kAxRun) * g.H;
       int vb = (vruns + 7) / 8;
       if (vb > 148 * 16) vb = 148 * 16;

@@ -45,6 +45,8 @@ struct CostArgs {
   int scale;
   int axis;                         // one other camera, axis-aligned flow matrix: zt.w holds 1/pz per plane
   int vcols;                        // axis, grey, scale 1: phase images as vertical triples, blocks from shared columns
+  int unit;                         // vcols and equal focal lengths: k_cost_unit (byte phase images, targets a whole shift away)
+  uint32_t norm_mul;                // unit: the normalised cost of a block sum S is (S · norm_mul) >> 8
   uint32_t one;                     // 1: a multiplier the compiler cannot fold, so that adds can issue on the FMA pipe
 };
 
@@ -135,6 +137,10 @@ void launch_phases(const CostArgs& a, cudaStream_t s);
 // Returns the kernel it used: 0 per-pixel warps, 1 per-row warps (uniform layers), 2 per-row warps of an axis-aligned pair.
 // Small layers with many planes: the warp-per-pixel cost kernel (and horizontal phase images) instead of the row kernels.
 bool cost_small_wide_layer(int W, int H, int n_planes);
+// The multiplier m with (S · m) >> 8 equal to the normalised cost of every grey block sum S (0..18) under `norm`, 0 if none.
+uint32_t cost_unit_norm(float norm);
+// Bytes of the byte phase images of a w x h camera (and the plane table behind them), for CostArgs::unit.
+size_t cost_unit_phase_bytes(int w, int h, int n_planes);
 int launch_cost(const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t* raw, int* err, cudaStream_t s);
 
 // sgm_emulate.cu: the exact replay of the reference's sheared-tile traversal on its line-buffer layout (any layer)
