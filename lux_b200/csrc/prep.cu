@@ -316,38 +316,54 @@ void launch_wta(const LayerGeom& g, const uint16_t* agg, float* depth, int* err,
 }
 
 // ---- DenseUpsampleLayer (DenseUpsampleLayer.cs:35-218) ----
-struct ShiftTaps {
-  float kx[4], ky[4];
-  int stepX, stepY;
-};
 
 // g2(x,y) = ImageShift(guide, 0.5, 0.5)(sx, sy) with the 16.16 nearest steps of NearestResize (:69-131): the shifted guide is
-// only ever read at these positions, so only they are computed.
-__global__ void k_shift_resize(const uint8_t* __restrict__ guide, int gw, int gh, int gstride, int pw, int ph, ShiftTaps t,
-                               uint8_t* __restrict__ g2) {
+// only ever read at these positions, so only they are computed. CubicTap (:56-62) of the half-pixel shift is exactly
+// (-1, 9, 9, -1) / 16 in both directions, so every product and sum of the two float passes is a multiple of 1/256 below 2^10,
+// exact in any order: they run on integers here, two channels a register vertically, and are rounded once (to even, as cvtps).
+// Bound by issue (some 200 operations a pixel): 2080x1560 of a 4160x3120 guide in 32 us; the float passes on byte loads took
+// 62 us, on word loads 56. WORDS: the guide's pixels are 4-byte aligned.
+template <bool WORDS>
+__global__ void __launch_bounds__(128) k_shift_resize(const uint8_t* __restrict__ guide, int gw, int gh, int gstride, int pw, int ph, int stepX,
+                                                      int stepY, uint8_t* __restrict__ g2) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= pw) return;
+  const int sx = (int)(((long long)stepX * x) >> 16);
+  int cols[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) cols[j] = min(max(sx - 1 + j, 0), gw - 1);  // clamp to edge
   for (int y = blockIdx.y; y < ph; y += gridDim.y) {  // gridDim.y is capped at 65535 rows; taller images loop
-  int sy = (int)((unsigned)y * (unsigned)t.stepY) >> 16;  // the accumulated yAcc (int, wraps like the reference's sum)
-  int sx = (int)((unsigned)x * (unsigned)t.stepX) >> 16;
-  int rows[4];
-  for (int i = 0; i < 4; i++) { int ry = sy - 1 + i; rows[i] = ry < 0 ? 0 : ry >= gh ? gh - 1 : ry; }
-  uint8_t outv[4];
-  for (int ch = 0; ch < 4; ch++) {
-    float v[4];
-    for (int j = 0; j < 4; j++) {  // columns sx-1 .. sx+2 of the row buffer (clamp-to-edge)
-      int c = sx - 1 + j;
-      int cx = c < 0 ? 0 : c >= gw ? gw - 1 : c;
-      float acc = __fmul_rn((float)guide[((size_t)rows[0] * gstride + cx) * 4 + ch], t.ky[0]);
-      for (int i = 1; i < 4; i++) acc = __fadd_rn(__fmul_rn((float)guide[((size_t)rows[i] * gstride + cx) * 4 + ch], t.ky[i]), acc);
-      v[j] = acc;
+    const int sy = (int)(((long long)stepY * y) >> 16);
+    uint32_t px[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const uint8_t* row = guide + (size_t)min(max(sy - 1 + i, 0), gh - 1) * gstride * 4;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const uint8_t* g = row + (size_t)cols[j] * 4;
+        if (WORDS) px[i][j] = __ldg(reinterpret_cast<const uint32_t*>(g));
+        else px[i][j] = g[0] | (uint32_t)g[1] << 8 | (uint32_t)g[2] << 16 | (uint32_t)g[3] << 24;
+      }
     }
-    float s = __fadd_rn(__fadd_rn(__fmul_rn(v[3], t.kx[3]), __fmul_rn(v[2], t.kx[2])),
-                        __fadd_rn(__fmul_rn(v[1], t.kx[1]), __fmul_rn(v[0], t.kx[0])));
-    int q = __float2int_rn(s);
-    outv[ch] = (uint8_t)(q < 0 ? 0 : q > 255 ? 255 : q);
-  }
-  *reinterpret_cast<uchar4*>(g2 + ((size_t)y * pw + x) * 4) = make_uchar4(outv[0], outv[1], outv[2], outv[3]);
+    uint32_t r[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {  // channels h and h + 2
+      uint32_t v[4];               // 16 x the column's value + 512, in 0 .. 5102
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        auto ch = [&](uint32_t w) { return __byte_perm(w, 0, h ? 0x4341 : 0x4240); };
+        v[j] = (ch(px[1][j]) + ch(px[2][j])) * 9u + 0x02000200u - (ch(px[0][j]) + ch(px[3][j]));
+      }
+      const uint32_t mid = v[1] + v[2], out = v[0] + v[3];
+      auto round256 = [](int n) {  // n/256 to the nearest, ties to even: in the low bits of 1.5·2^23 + n/256
+        const float f = __fsub_rn(__int_as_float(0x4b400000 + n), 12582912.0f);
+        return __float_as_uint(__fmaf_rn(f, 1.0f / 256.0f, 12582912.0f));
+      };
+      const uint32_t lo = round256((int)((mid & 0xffffu) * 9u - (out & 0xffffu)) - 8192);
+      const uint32_t hi = round256((int)((mid >> 16) * 9u - (out >> 16)) - 8192);
+      r[h] = __vmins2(__vmaxs2(__byte_perm(lo, hi, 0x5410), 0u), 0x00ff00ffu);
+    }
+    reinterpret_cast<uint32_t*>(g2)[(size_t)y * pw + x] = r[0] | r[1] << 8;
   }
 }
 
@@ -361,19 +377,52 @@ LUX_DEV float up_exp2(float t) {  // Exp2Fast (:151-159)
   float p = __fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(__fadd_rn(__fmul_rn(f, C1), C2), f), C3), f), C4);
   return __uint_as_float(__float_as_uint(p) + ((unsigned)n << 23));
 }
+// Two floats a register pair, each operation rounded as its scalar form.
+struct F2 {
+  uint64_t v;
+};
+LUX_DEV F2 f2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b)); return r; }
+LUX_DEV void f2_get(F2 p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p.v)); }
+LUX_DEV F2 operator+(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+LUX_DEV F2 operator*(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+// a·b for a sum that follows: a pair's mul.rn is contracted with the add.rn that takes its product, in spite of --fmad=false.
+// minus0 is (-0.0, -0.0) in a form that the compiler does not see through: a kernel argument.
+LUX_DEV F2 mul_alone(F2 a, F2 b, F2 minus0) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(minus0.v));
+  return r;
+}
+LUX_DEV F2 add_up(F2 a, F2 b) { F2 r; asm("add.rp.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+LUX_DEV F2 f2_neg(F2 a) { return F2{a.v ^ 0x8000000080000000ull}; }
+
+// up_exp2 of two t <= -0.0, given as -t, without conversions: there n = ceil(t) - 1, and t + M rounded up holds ceil(t) in its
+// low bits. M = 1.5·2^23 + 511, whose bits end in 511, so a shift of the sum's bits by 23 leaves n alone. t - n is rounded
+// once as there: the sum's difference to M + 1 is whole and exact.
+LUX_DEV F2 up_exp2_neg(float a, float b, F2 minus0) {
+  const float C1 = __uint_as_float(0x3d9fcb52u), C2 = __uint_as_float(0x3e677e26u), C3 = __uint_as_float(0x3f322226u),
+              C4 = __uint_as_float(0x3f7ffb19u), M = 12583423.0f;
+  const F2 t = f2(-fminf(a, 126.0f), -fminf(b, 126.0f));
+  const F2 m = add_up(t, f2(M, M)), f = t + (f2(M + 1.0f, M + 1.0f) + f2_neg(m));
+  F2 p = mul_alone(f, f2(C1, C1), minus0) + f2(C2, C2);
+  p = mul_alone(p, f, minus0) + f2(C3, C3);
+  p = mul_alone(p, f, minus0) + f2(C4, C4);
+  float p0, p1, m0, m1;
+  f2_get(p, p0, p1);
+  f2_get(m, m0, m1);
+  return f2(__uint_as_float(__float_as_uint(p0) + (__float_as_uint(m0) << 23)), __uint_as_float(__float_as_uint(p1) + (__float_as_uint(m1) << 23)));
+}
+// Byte c of w as 2^23 + byte: a permute, where a conversion has a quarter of its rate.
+LUX_DEV float byte_bias(uint32_t w, int c) { return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440 | c)); }
 LUX_DEV float spatial_w(float f, int i) {  // SpatialW (:212-217)
   float d = fabsf(__fsub_rn(f, (float)(i * 2)));
   d = d < 1.0f ? d : 1.0f;
   return f2i(d) == 0 ? 1.0f : __uint_as_float(0x3eaaaaabu);
 }
 
-// BilateralUpsampleFromCollapse (:166-209). inverse != 0: lo = rcp(prev) and out = rcp(V/S) (the InverseDepth steps).
-__global__ void k_bilateral(const float* __restrict__ prev, int lw, int lh, const uint8_t* __restrict__ guide, int W, int H, int gstride,
-                            const uint8_t* __restrict__ g2, float k, int inverse, const uint32_t* __restrict__ rcp_table,
-                            float* __restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= W) return;
-  for (int y = blockIdx.y; y < H; y += gridDim.y) {  // gridDim.y is capped at 65535 rows; taller images loop
+// BilateralUpsampleFromCollapse (:166-209) for one output pixel. inverse: lo = rcp(prev) and out = rcp(V/S) (the InverseDepth
+// steps).
+LUX_DEV float bilateral_pixel(const float* __restrict__ prev, int lw, int lh, const uint8_t* __restrict__ guide, int gstride,
+                              const uint8_t* __restrict__ g2, float k, bool inverse, const uint32_t* __restrict__ rcp_table, int x, int y) {
   const float eps = __uint_as_float(0x322bcc77u);
   int wm1 = lw - 1, hm1 = lh - 1;
   int iy0 = (y - 1) / 2;
@@ -412,46 +461,152 @@ __global__ void k_bilateral(const float* __restrict__ prev, int lw, int lh, cons
     accV = __fadd_rn(v1, __fadd_rn(v0, accV));
     accS = __fadd_rn(w1, __fadd_rn(w0, accS));
   }
-  float r = __fdiv_rn(accV, accS);
-  out[(size_t)y * W + x] = inverse ? rcp_approx(r, rcp_table) : r;
+  const float r = __fdiv_rn(accV, accS);
+  return inverse ? rcp_approx(r, rcp_table) : r;
+}
+
+// What one upsample reads and writes: the depth and, where conf is not null, the confidence.
+struct Bilateral {
+  const float *prev, *conf;
+  int lw, lh;
+  const uint8_t* guide;
+  int W, H, gstride;
+  const uint8_t* g2;
+  float k;
+  const uint32_t* rcp;
+  float *out, *out_conf;
+  int qx, qy;  // quads: output pixels 1..2·qx by 1..2·qy
+  uint64_t minus0;  // for mul_alone
+};
+
+// The output pixels outside the quads, one by one: row 0 and the rows past the quads, then column 0 and the columns past
+// them.
+__global__ void k_bilateral_border(const Bilateral b) {
+  const int top = b.H - 2 * b.qy, side = b.W - 2 * b.qx;  // rows and columns outside the quads
+  const size_t n = (size_t)top * b.W + (size_t)side * 2 * b.qy;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    int x, y;
+    if (i < (size_t)top * b.W) {
+      const int r = (int)(i / b.W);
+      x = (int)(i - (size_t)r * b.W);
+      y = r == 0 ? 0 : 2 * b.qy + r;
+    } else {
+      const size_t j = i - (size_t)top * b.W;
+      const int r = (int)(j / side), c = (int)(j - (size_t)r * side);
+      y = 1 + r;
+      x = c == 0 ? 0 : 2 * b.qx + c;
+    }
+    b.out[(size_t)y * b.W + x] = bilateral_pixel(b.prev, b.lw, b.lh, b.guide, b.gstride, b.g2, b.k, true, b.rcp, x, y);
+    if (b.conf) b.out_conf[(size_t)y * b.W + x] = bilateral_pixel(b.conf, b.lw, b.lh, b.guide, b.gstride, b.g2, b.k, false, b.rcp, x, y);
   }
 }
 
-static float cubic_tap_host(float x) {  // CubicTap (:56-62)
-  uint32_t u = 0x3e2aaaabu;
-  float sixth;
-  memcpy(&sixth, &u, 4);
-  volatile float x2 = x * x, x3 = x2 * x;
-  if (x < 1.0f) { volatile float a = x3 * 9.0f; volatile float b = x2 * (-15.0f); b = b + 6.0f; b = b + a; return b * sixth; }
-  if (x < 2.0f) {
-    volatile float a = x3 * (-3.0f); volatile float b = x2 * 15.0f; volatile float c = x * (-24.0f);
-    c = c + 12.0f; c = c + b; c = c + a; return c * sixth;
+// Output pixels 2i + 1 and 2i + 2 of rows 2j + 1 and 2j + 2 share their four low-resolution pixels (i, i + 1) x (j, j + 1): a
+// thread makes the four, loading and inverting the low pixels once, and the confidence with the depth's weights. The
+// spatial weights are then 1 for the nearer column or row and a third for the farther one. The two taps of a row run in one
+// register pair. Persistent blocks, as many as are resident, with the rcpps table in shared memory. Bound by issue: depth and
+// confidence of 4160x3120 88 us; scalar taps took 128, one thread an output pixel and a launch each 297.
+constexpr int kQuadBlocks = 5;  // of 256 threads an SM, by their registers
+template <bool CONF>
+__global__ void __launch_bounds__(256, kQuadBlocks) k_bilateral_quads(const Bilateral b) {
+  __shared__ uint32_t tab[4096];
+  for (int i = threadIdx.x; i < 1024; i += 256) reinterpret_cast<uint4*>(tab)[i] = __ldg(reinterpret_cast<const uint4*>(b.rcp) + i);
+  __syncthreads();
+  auto rcp = [&](float v) {  // rcp_entry, as selections
+    const uint32_t u = fbits(v), r = tab[(u >> 11) & 0xfff], sign = u & 0x80000000u, a = u & 0x7fffffffu;
+    const int re = (int)((r >> 23) & 0xff) + 127 - (int)(a >> 23);
+    uint32_t o = sign | (re > 0 ? (uint32_t)re << 23 | (r & 0x7fffffu) : 0u);
+    o = a < 0x800000u ? sign | 0x7f800000u : o;
+    return ffrom(a < 0x7f800000u ? o : a == 0x7f800000u ? sign : u | 0x400000u);
+  };
+  const float eps = __uint_as_float(0x322bcc77u), third = __uint_as_float(0x3eaaaaabu), third2 = __fmul_rn(third, third);
+  const F2 near_far[2][2] = {{f2(1.0f, third), f2(third, 1.0f)}, {f2(third, third2), f2(third2, third)}};
+  const unsigned n = (unsigned)b.qx * (unsigned)b.qy, step = gridDim.x * 256u;
+  for (unsigned t = blockIdx.x * 256u + threadIdx.x; t < n; t += step) {
+    const int j = (int)(t / (unsigned)b.qx), i = (int)(t - (unsigned)j * (unsigned)b.qx);
+    F2 lo[2], cf[2], q[2][3];  // low pixels (0, r), (1, r); the guide's negated
+    uint32_t hw[4];
+#pragma unroll
+    for (int o = 0; o < 4; o++)
+      hw[o] = __ldg(reinterpret_cast<const uint32_t*>(b.guide) + (2 * (size_t)j + 1 + (o >> 1)) * b.gstride + 2 * i + 1 + (o & 1));
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const size_t p = (size_t)(j + r) * b.lw + i;
+      lo[r] = f2(rcp(__ldg(b.prev + p)), rcp(__ldg(b.prev + p + 1)));
+      if (CONF) cf[r] = f2(__ldg(b.conf + p), __ldg(b.conf + p + 1));
+      const uint32_t w0 = __ldg(reinterpret_cast<const uint32_t*>(b.g2) + p), w1 = __ldg(reinterpret_cast<const uint32_t*>(b.g2) + p + 1);
+#pragma unroll
+      for (int ch = 0; ch < 3; ch++) q[r][ch] = f2(-byte_bias(w0, ch), -byte_bias(w1, ch));
+    }
+#pragma unroll
+    for (int o = 0; o < 4; o++) {  // the output pixel (o & 1, o >> 1) of the quad
+      float accV = 0.0f, accS = 0.0f, accC = 0.0f;
+#pragma unroll
+      for (int r = 0; r < 2; r++) {
+        F2 d[3];
+#pragma unroll
+        for (int ch = 0; ch < 3; ch++) {
+          const float h = byte_bias(hw[o], ch);  // both sides of the difference carry the 2^23
+          d[ch] = f2(h, h) + q[r][ch];
+          d[ch] = d[ch] * d[ch];  // (whole numbers below 2^18 in all: no rounding)
+        }
+        float e0, e1, w0, w1, v0, v1;
+        f2_get((d[1] + (d[2] + d[0])) * f2(b.k, b.k), e0, e1);
+        const F2 wt = (up_exp2_neg(e0, e1, F2{b.minus0}) + f2(eps, eps)) * near_far[(o >> 1) != r][o & 1];
+        f2_get(lo[r] * wt, v0, v1);
+        accV = __fadd_rn(v1, __fadd_rn(v0, accV));
+        if (CONF) {
+          f2_get(cf[r] * wt, v0, v1);
+          accC = __fadd_rn(v1, __fadd_rn(v0, accC));
+        }
+        f2_get(wt, w0, w1);
+        accS = __fadd_rn(w1, __fadd_rn(w0, accS));
+      }
+      const size_t at = (2 * (size_t)j + 1 + (o >> 1)) * b.W + 2 * i + 1 + (o & 1);
+      b.out[at] = rcp(__fdiv_rn(accV, accS));
+      if (CONF) b.out_conf[at] = __fdiv_rn(accC, accS);
+    }
   }
-  return 0.0f;
 }
 
 void launch_upsample(const float* prev, int pw, int ph, const uint8_t* guide, int gw, int gh, int gstride, float sigma,
                      const uint32_t* rcp_table, uint8_t* g2, float* out_depth, const float* prev_conf, float* out_conf,
                      cudaStream_t s) {
-  ShiftTaps t;
-  float tx = 0.5f, ty = 0.5f;  // ImageShift(guide, 0.5f, 0.5f): floor 0, fraction 0.5
-  t.kx[0] = cubic_tap_host(tx + 1.0f); t.kx[1] = cubic_tap_host(tx); t.kx[2] = cubic_tap_host(1.0f - tx); t.kx[3] = cubic_tap_host(2.0f - tx);
-  t.ky[0] = cubic_tap_host(ty + 1.0f); t.ky[1] = cubic_tap_host(ty); t.ky[2] = cubic_tap_host(1.0f - ty); t.ky[3] = cubic_tap_host(2.0f - ty);
   double sy = (double)gh * 65536.0 / (double)ph, sx = (double)gw * 65536.0 / (double)pw;
-  t.stepY = sy >= 2147483648.0 ? 0x7fffffff : (int)sy;
-  t.stepX = sx >= 2147483648.0 ? 0x7fffffff : (int)sx;
+  const int stepY = sy >= 2147483648.0 ? 0x7fffffff : (int)sy;
+  const int stepX = sx >= 2147483648.0 ? 0x7fffffff : (int)sx;
   dim3 g1((pw + 127) / 128, std::min(ph, 65535));
-  k_shift_resize<<<g1, 128, 0, s>>>(guide, gw, gh, gstride, pw, ph, t, g2);
-  count_launches(1);
+  const bool words = (reinterpret_cast<uintptr_t>(guide) & 3) == 0;  // a caller's guide may lie at any address
+  if (words) k_shift_resize<true><<<g1, 128, 0, s>>>(guide, gw, gh, gstride, pw, ph, stepX, stepY, g2);
+  else k_shift_resize<false><<<g1, 128, 0, s>>>(guide, gw, gh, gstride, pw, ph, stepX, stepY, g2);
   volatile float ss = sigma * sigma;
-  float k = 0.5f / ss;
-  dim3 g3((gw + 127) / 128, std::min(gh, 65535));
-  k_bilateral<<<g3, 128, 0, s>>>(prev, pw, ph, guide, gw, gh, gstride, g2, k, 1, rcp_table, out_depth);
-  count_launches(1);
-  if (prev_conf && out_conf) {
-    k_bilateral<<<g3, 128, 0, s>>>(prev_conf, pw, ph, guide, gw, gh, gstride, g2, k, 0, rcp_table, out_conf);
-    count_launches(1);
+  Bilateral b;
+  b.prev = prev; b.lw = pw; b.lh = ph; b.guide = guide; b.W = gw; b.H = gh; b.gstride = gstride; b.g2 = g2;
+  b.k = 0.5f / ss;
+  b.rcp = rcp_table;
+  b.out = out_depth;
+  b.conf = prev_conf && out_conf ? prev_conf : nullptr;
+  b.out_conf = out_conf;
+  b.minus0 = 0x8000000080000000ull;
+  // the quads whose four low pixels exist; their exponents are <= -0.0 for a positive finite k, float holds their coordinates
+  // exactly below 2^23, and a 32-bit index counts them
+  const bool quads = words && b.k > 0.0f && b.k <= 3.4e38f && gw < (1 << 23) && gh < (1 << 23) && (size_t)pw * ph < ((size_t)1 << 31);
+  b.qx = quads ? std::max(0, std::min((gw - 1) / 2, pw - 1)) : 0;
+  b.qy = quads ? std::max(0, std::min((gh - 1) / 2, ph - 1)) : 0;
+  if (b.qx == 0 || b.qy == 0) b.qx = b.qy = 0;
+  int launches = 1;
+  if (b.qx > 0) {
+    const unsigned grid = (unsigned)std::min<size_t>(((size_t)b.qx * b.qy + 255) / 256, 148 * kQuadBlocks);
+    if (b.conf) k_bilateral_quads<true><<<grid, 256, 0, s>>>(b);
+    else k_bilateral_quads<false><<<grid, 256, 0, s>>>(b);
+    launches++;
   }
+  const size_t rest = (size_t)(gh - 2 * b.qy) * gw + (size_t)(gw - 2 * b.qx) * 2 * b.qy;
+  if (rest > 0) {
+    k_bilateral_border<<<(unsigned)std::min<size_t>((rest + 127) / 128, 148 * 64), 128, 0, s>>>(b);
+    launches++;
+  }
+  count_launches(launches);
 }
 
 }  // namespace lux

@@ -1,0 +1,47 @@
+"""The upsample by quads of output pixels (four that share their low-resolution pixels) and the border pixel by pixel, against the
+oracle bit for bit: sizes without quads, with one, around a block's 256 quads; with and without confidence; a guide at an odd address; exponents beyond the range that the weights clamp, and depths whose reciprocal is not a normal number."""
+import ctypes
+
+import numpy as np
+import pytest
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pw,ph,gw,gh,with_conf,sigma", [
+    (1, 1, 2, 2, True, 10.0), (2, 2, 4, 4, True, 10.0), (2, 9, 4, 18, False, 10.0), (3, 2, 6, 4, True, 0.5), (257, 2, 514, 4, False, 10.0),
+    (17, 17, 34, 34, True, 1e-3), (16, 16, 32, 32, False, 300.0), (129, 31, 258, 62, True, 10.0)])
+def test_quads(oracle, pw, ph, gw, gh, with_conf, sigma):
+    from lux_b200 import api
+    rng = np.random.default_rng(pw * 100 + ph)
+    depth = rng.uniform(300.0, 6000.0, (ph, pw)).astype(np.float32)
+    depth.reshape(-1)[::7] = [np.float32(v) for v in np.resize([0.0, -0.0, np.inf, 1e-40, 3e38, -5.0], depth.reshape(-1)[::7].size)]
+    guide = rng.integers(0, 256, (gh, gw, 4), dtype=np.uint8)
+    guide[: gh // 2] = 255  # flat: every weight's exponent is -0
+    conf = rng.uniform(0, 1, (ph, pw)).astype(np.float32) if with_conf else None
+    od, oc = oracle.upsample(depth, pw, ph, guide, pw, ph, sigma=sigma, prev_conf=conf)
+    r = api.DenseUpsampleLayer.run(depth, pw, ph, guide, pw, ph, sigma=sigma, prev_confidence=conf)
+    same = (r.Depth.reshape(od.shape).view(np.uint32) == od.view(np.uint32)) | (np.isnan(od) & np.isnan(r.Depth.reshape(od.shape)))
+    assert same.all()
+    if with_conf:
+        assert np.array_equal(r.Confidence.reshape(oc.shape).view(np.uint32), oc.view(np.uint32))
+
+
+@pytest.mark.gpu
+def test_guide_at_an_odd_address(oracle):
+    import torch
+    from lux_b200 import _lib, api
+    pw, ph = 33, 9
+    rng = np.random.default_rng(5)
+    depth = rng.uniform(300.0, 6000.0, (ph, pw)).astype(np.float32)
+    guide = rng.integers(0, 256, (2 * ph, 2 * pw, 4), dtype=np.uint8)
+    ctx = api.default_context()
+    d_prev = torch.from_numpy(depth).cuda()
+    d_guide = torch.zeros(guide.size + 16, dtype=torch.uint8, device="cuda")
+    d_guide[1:1 + guide.size] = torch.from_numpy(guide.reshape(-1)).cuda()
+    d_out = torch.zeros(2 * ph, 2 * pw, device="cuda")
+    torch.cuda.synchronize()
+    img = _lib.Img(d_guide.data_ptr() + 1, 2 * pw, 2 * ph, 2 * pw, 1)
+    ctx.check(ctx.lib.lux_sgm_upsample_noalloc(ctx.handle, d_prev.data_ptr(), pw, ph, ctypes.byref(img), pw, ph, 12.0, 2, None,
+                                               d_out.data_ptr(), None))
+    od, _ = oracle.upsample(depth, pw, ph, guide, pw, ph)
+    assert np.array_equal(d_out.cpu().numpy().view(np.uint32), od.view(np.uint32))
