@@ -672,9 +672,8 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
   for (int seg = nseg - 1; seg >= 0; seg--) {
     const int t0 = seg * kSeg;
     cp_async_wait<0>();
-    // a whole segment clear of the line's last pixel (where its backward walk starts; a warp's lines may differ by one step)
-    // and of the sides (a new line; column 1, where pass -1's states are kept)
-    bool odd = t0 + kSeg >= NS;
+    // a whole segment clear of the sides (a new line; column 1, where pass -1's states are kept)
+    bool odd = t0 + kSeg > NS;
     if (P == 1) odd |= x0 <= 1 || x0 + kSeg >= W;
     if (P == 3) odd |= x0 == W - 1 || x0 < kSeg;
     if (P == 0) odd |= t0 <= 1;

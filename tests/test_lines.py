@@ -89,19 +89,3 @@ def test_lines_yields_to_pass1_and_chosen_forms(ctx):
     finally:
         api.set_tuned_form(123, 77, 40, 16, 0)
     assert _solve(ctx, wl)[0] == LINES
-
-
-@pytest.mark.parametrize("w,h,d,tile", [(1501, 1313, 128, 64), (1601, 1321, 120, 32)])
-def test_lines_of_a_warp_end_a_step_apart(ctx, w, h, d, tile):
-    """A warp of the large form holds diagonals of 8k + 1 and 8k steps: the shorter one's last segment is whole."""
-    from lux_b200 import synth
-    step, px = w + 1, w * h
-    lens = [(px - r + step - 1) // step for r in range(step)]
-    assert any(lens[r] != lens[r + 1] and lens[r + 1] % 8 == 0 for r in range(0, step - 1, 2)) and px * d >= 240 << 20
-    wl = synth.rectified_pair(w, h, d, seed=13, tile=tile)
-    form, agg, depth = _solve(ctx, wl, keep_agg=True)
-    assert form == LINES
-    form, agg2, depth2 = _solve(ctx, wl, keep_agg=True, sgm="split")
-    assert form == 2
-    assert np.array_equal(agg, agg2)
-    assert np.array_equal(depth.view(np.uint32), depth2.view(np.uint32))
