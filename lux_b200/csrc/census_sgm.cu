@@ -6,10 +6,13 @@
 // median fusion) are spelled out with each kernel.
 //
 // Layout in HBM: census images W x H uint64; the cost volume [pixel][Dp] uint8 and the path sums [pixel][Dp] uint16 with
-// Dp = 32 x LPT >= D (disparities over the 32 lanes of a warp, LPT per lane).
+// Dp = 32 x LPT >= D (LPT = 1, 2, 4 or 8). The sums that the lines leave keep lines.cuh's order within every octet.
+#include <algorithm>
+
 #include "../../include/lux_sgm.h"
 #include "common.cuh"
 #include "internal.h"
+#include "lines.cuh"
 
 namespace lux {
 
@@ -28,8 +31,19 @@ LUX_DEV uint32_t pick(const uint32_t (&v)[LPT], int i) {
   return r;
 }
 
-// The first disparity with the least path sum S[0..D) of a pixel held by a warp (LPT a lane), with the parabolic subpixel
-// correction (S[d-1] - S[d+1]) / (2 (S[d-1] - 2 S[d] + S[d+1])) where 0 < d < D - 1 and the denominator is positive.
+// Disparity d of least sum b with the parabolic subpixel correction (a - c) / (2 (a - 2 b + c)), a and c the sums beside it,
+// where 0 < d < D - 1 and the denominator is positive.
+LUX_DEV float refine(int d, int D, int subpixel, float b, float a, float c) {
+  float out = (float)d;
+  if (subpixel && d > 0 && d < D - 1) {
+    const float den = __fmul_rn(2.0f, __fadd_rn(__fsub_rn(a, __fmul_rn(2.0f, b)), c));
+    if (den > 0.0f) out = __fadd_rn(out, __fdiv_rn(__fsub_rn(a, c), den));
+  }
+  return out;
+}
+LUX_DEV int octet_pos(int k) { return 2 * (k & 3) + (k >> 2); }  // where the lines keep plane k of an octet
+
+// The first disparity with the least path sum S[0..D) of a pixel held by a warp (LPT a lane), refined.
 template <int LPT>
 LUX_DEV void wta_of(const uint32_t (&s)[LPT], int lane, int D, int subpixel, int& d_out, float& disp_out) {
   uint32_t best = kBig, arg = kBig;
@@ -47,14 +61,8 @@ LUX_DEV void wta_of(const uint32_t (&s)[LPT], int lane, int D, int subpixel, int
   const int dm = max(d - 1, 0), dp = min(d + 1, D - 1);
   const float a = (float)__shfl_sync(0xffffffffu, pick<LPT>(s, dm % LPT) & 0xffffu, dm / LPT);
   const float c = (float)__shfl_sync(0xffffffffu, pick<LPT>(s, dp % LPT) & 0xffffu, dp / LPT);
-  float out = (float)d;
-  if (subpixel && d > 0 && d < D - 1) {
-    const float b = (float)m;
-    const float den = __fmul_rn(2.0f, __fadd_rn(__fsub_rn(a, __fmul_rn(2.0f, b)), c));
-    if (den > 0.0f) out = __fadd_rn(out, __fdiv_rn(__fsub_rn(a, c), den));
-  }
   d_out = d;
-  disp_out = out;
+  disp_out = refine(d, D, subpixel, (float)m, a, c);
 }
 
 // Bit k (row-major over the window, centre skipped) is set when that neighbour, read at the clamped position, is darker
@@ -253,8 +261,294 @@ __global__ void __launch_bounds__(128) k_census_path(const CensusPairs ps, int w
   }
 }
 
-// The right image's first minimum over d of S(x + d, y, d), x + d < W (a warp per right-image pixel).
-template <int LPT>
+// The paths along single lines, as k_lines_walk of sgm_lines.cu walks them, without its revisits and with constant penalties:
+// a lane holds eight disparities as u16 pairs, a line takes GL = Dp / 8 lanes, the forward states are kept every kSeg pixels
+// and the pair walk of a path shares its launch with the forward walk of the next. A line starts from L = 0 (its first step
+// is then L = C). Disparities past D cost kBeyond more than their byte: they stay above every true L (62 + P2 <= 8191), and
+// above m + P2 also as neighbours. Their sums may wrap: the high half of a pair never carries into a true one (plane p + 4
+// is past D where plane p is), and the winner-take-all takes them as 0xffff (eight true L sum up to 65528 at most).
+// The eight walks of one disparity a lane, one warp a line and one pixel of prefetch took 10.4 ms at 2080x1560 D=128 (each
+// was bound by its steps' latency, at 1.2 TB/s); these take 3.5 ms.
+constexpr uint32_t kBeyond = 0x40004000u;
+
+struct CensusLines {
+  int W, H, n;  // n: Dp
+  uint32_t p1x2, p2x2, one;
+  int subpixel, keep;  // keep: the sums are read again
+  uint16_t *ckpt, *ckpt_min;  // per pair of the launch [2][states][n] and [2][states], even and odd paths
+  size_t states;
+  CensusPairs ps;
+};
+
+// unpack8 with the disparities past D raised by kBeyond
+LUX_DEV void unpack_cost(L4& v, uint2 b, const L4& pad) {
+  unpack8(v, b);
+#pragma unroll
+  for (int k = 0; k < 4; k++) v.r[k] |= pad.r[k];
+}
+LUX_DEV L4 pad_of(int gl, int D, uint32_t value) {
+  L4 v;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    v.r[k] = (gl * 8 + k >= D ? value & 0xffffu : 0u) | (gl * 8 + k + 4 >= D ? value & 0xffff0000u : 0u);
+  return v;
+}
+LUX_DEV void set_zero(L4& v, uint32_t& md) { v.r[0] = v.r[1] = v.r[2] = v.r[3] = md = 0; }
+
+template <int GL, int P>
+LUX_DEV void census_forward(const CensusLines& a, const CensusPair& pr, int wi, uint2* ring, uint16_t* ckpt, uint16_t* ckpt_min) {
+  constexpr int LPW = 32 / GL;
+  static_assert(kBatch == kSeg, "one state a batch");
+  const int n = a.n, lane = threadIdx.x & 31, gl = lane & (GL - 1), grp = lane / GL;
+  const int NL = line_count(a, P);
+  if (wi * LPW >= NL) return;
+  const int line0 = wi * LPW + grp, line = min(line0, NL - 1);
+  const bool in = line0 < NL, first = gl == 0, last = gl == GL - 1;
+  const int NS = line_len(a, P, line);
+  Walk w = walk_at(a, P, line_first(a, P, line), 1), ws = w;
+  const L4 pad = pad_of(gl, pr.D, kBeyond);
+  RawRing rr(ring + lane, in);
+  L4 L;
+  uint32_t md;
+  set_zero(L, md);
+  const int steps = __reduce_max_sync(0xffffffffu, NS), nb = (steps + kBatch - 1) / kBatch;
+  stage_batch(rr, 0, pr.cost, n, ws, NS, gl, in);
+  ws.advance();
+  stage_batch(rr, 1, pr.cost, n, ws, NS - kBatch, gl, in);
+  ws.advance();
+  for (int b = 0; b + 1 < nb; b++) {  // (no state is kept after the last batch)
+    cp_async_wait<1>();
+    bool odd = (b + 1) * kBatch > NS;  // else a whole batch without a new line
+    if (P == 1) odd |= w.x == 0 || w.x + kBatch > a.W;
+    if (P == 3) odd |= w.x == a.W - 1 || w.x + 1 < kBatch;
+    if (!__any_sync(0xffffffffu, odd)) {
+      uint2 rb[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) rb[i] = rr.get(b, i);
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) {
+        L4 raw2;
+        unpack_cost(raw2, rb[i], pad);
+        line_step<GL, kBeyond>(L, md, raw2, a.p2x2, a, first, last);
+      }
+    } else {
+      int x = w.x;
+#pragma unroll 1
+      for (int i = 0; i < kBatch; i++) {
+        if ((P == 1 && x == 0) || (P == 3 && x == a.W - 1)) set_zero(L, md);
+        L4 raw2;
+        unpack_cost(raw2, rr.get(b, i), pad);
+        line_step<GL, kBeyond>(L, md, raw2, a.p2x2, a, first, last);
+        x += w.dx;
+        if ((unsigned)x >= (unsigned)a.W) x -= w.dx * a.W;
+      }
+    }
+    if (in && (b + 1) * kSeg < NS) {
+      const size_t ci = (size_t)b * NL + line;
+      __stcs(reinterpret_cast<uint4*>(ckpt + ci * n) + gl, as_uint4(L));
+      if (gl == 0) ckpt_min[ci] = (uint16_t)(md & 0xffffu);
+    }
+    w.advance();
+    stage_batch(rr, b + 2, pr.cost, n, ws, NS - (b + 2) * kBatch, gl, in);
+    ws.advance();
+  }
+  cp_async_wait<0>();
+}
+
+// MODE 0 stores the sums, 1 adds to them, 2 adds, stores them where they are kept, and takes the winner.
+template <int GL, int P, int MODE>
+LUX_DEV void census_pair(const CensusLines& a, const CensusPair& pr, int wi, uint4* sum, uint2* rawp, const uint16_t* ckpt,
+                         const uint16_t* ckpt_min) {
+  constexpr int LPW = 32 / GL, dx = P == 1 ? 1 : P == 3 ? -1 : 0, PX = GL < kSeg ? kSeg / GL : 1;  // PX: a segment's pixels a lane
+  const int W = a.W, n = a.n, lane = threadIdx.x & 31, gl = lane & (GL - 1), grp = lane / GL;
+  const int NL = line_count(a, P);
+  if (wi * LPW >= NL) return;
+  const int line0 = wi * LPW + grp, line = min(line0, NL - 1);
+  const bool in = line0 < NL, first = gl == 0, last = gl == GL - 1;
+  const int NS = line_len(a, P, line), step = line_step_of(P, W);
+  const int steps = __reduce_max_sync(0xffffffffu, NS), nseg = (steps + kSeg - 1) / kSeg;
+  const L4 pad = pad_of(gl, pr.D, kBeyond);
+  sum += lane;
+  rawp += lane;
+  if (!in)
+    for (int i = 0; i < kSeg; i++) rawp[i * 32] = kPastRaw;
+  int pi0 = line_first(a, P, line) + (nseg - 1) * kSeg * step, x0 = dx != 0 ? pi0 % W : 0;  // of the segment in hand
+  auto stage = [&](int i, int pi) {
+    if (MODE != 0) cp_async16(sum + i * 32, reinterpret_cast<const uint4*>(pr.S + (size_t)pi * n) + gl);
+    cp_async8(rawp + i * 32, reinterpret_cast<const uint2*>(pr.cost + (size_t)pi * n) + gl);
+  };
+  for (int i = 0; i < kSeg; i++)
+    if (in && (nseg - 1) * kSeg + i < NS) stage(i, pi0 + step * i);
+  cp_async_commit();
+  auto load_ckpt = [&](int seg, L4& L, uint32_t& mn) {  // the forward state before segment seg, its minimum not yet doubled
+    set_zero(L, mn);
+    if (seg > 0 && seg * kSeg < NS && in) {
+      const size_t ci = (size_t)(seg - 1) * NL + line;
+      L = as_l4(__ldcs(reinterpret_cast<const uint4*>(ckpt + ci * n) + gl));
+      mn = __ldcs(ckpt_min + ci);
+    }
+  };
+  L4 F, B;  // the forward and backward states
+  uint32_t fd, bd;
+  load_ckpt(nseg - 1, F, fd);
+  fd = dup16(fd);
+  set_zero(B, bd);
+  for (int seg = nseg - 1; seg >= 0; seg--) {
+    const int t0 = seg * kSeg;
+    cp_async_wait<0>();
+    // a whole segment clear of new lines either way (where two lines of a warp end a step apart, one of
+    // them is at a side in the segment in which the shorter one ends)
+    bool odd = t0 + kSeg > NS;
+    if (P == 1) odd |= x0 == 0 || x0 + kSeg >= W;
+    if (P == 3) odd |= x0 == W - 1 || x0 < kSeg;
+    const bool plain = seg > 0 && !__any_sync(0xffffffffu, odd);
+    auto add_fwd = [&](int i) {
+      if (MODE == 0) {
+        sum[i * 32] = as_uint4(F);
+      } else {
+        uint4 s = sum[i * 32];
+        s.x += F.r[0];
+        s.y += F.r[1];
+        s.z += F.r[2];
+        s.w += F.r[3];
+        sum[i * 32] = s;
+      }
+    };
+    if (plain) {
+#pragma unroll
+      for (int i = 0; i < kSeg; i++) {
+        L4 raw2;
+        unpack_cost(raw2, rawp[i * 32], pad);
+        line_step<GL, kBeyond>(F, fd, raw2, a.p2x2, a, first, last);
+        add_fwd(i);
+      }
+    } else {
+      int x = x0;
+#pragma unroll 1
+      for (int i = 0; i < kSeg; i++) {
+        if ((P == 1 && x == 0) || (P == 3 && x == W - 1)) set_zero(F, fd);
+        L4 raw2;
+        unpack_cost(raw2, rawp[i * 32], pad);
+        line_step<GL, kBeyond>(F, fd, raw2, a.p2x2, a, first, last);
+        add_fwd(i);
+        x += dx;
+        if ((unsigned)x >= (unsigned)W) x -= dx * W;
+      }
+    }
+    const int pq = pi0 - step * kSeg;  // the segment before
+    L4 Fn;
+    uint32_t fdn;
+    load_ckpt(seg - 1, Fn, fdn);
+    // lane i (mod GL): the segment's pixels i, i + GL: the winner, its sum, and the sums beside it (low and high half)
+    int win[PX] = {};
+    uint32_t least[PX] = {}, beside[PX] = {};
+    auto put = [&](int i, int pi, bool live) {
+      L4 s = as_l4(sum[i * 32]);
+#pragma unroll
+      for (int k = 0; k < 4; k++) s.r[k] += B.r[k];
+      if ((MODE != 2 || a.keep) && in && live) __stcs(reinterpret_cast<uint4*>(pr.S + (size_t)pi * n) + gl, as_uint4(s));
+      if constexpr (MODE == 2) {
+        const L4 full = pad_of(gl, pr.D, 0xffffffffu);
+#pragma unroll
+        for (int k = 0; k < 4; k++) s.r[k] |= full.r[k];
+        const int arg = wta_line<GL>(s, gl, lane, true);
+        sum[i * 32] = as_uint4(s);
+        __syncwarp();
+        const uint16_t* sums = reinterpret_cast<const uint16_t*>(sum + i * 32 - gl);
+        auto at = [&](int d) { return (uint32_t)sums[(d & ~7) + octet_pos(d & 7)]; };
+        if ((gl & (kSeg - 1)) == (i & (GL - 1) & (kSeg - 1))) {
+          const uint32_t m = at(arg), bs = at(max(arg - 1, 0)) | at(min(arg + 1, pr.D - 1)) << 16;
+#pragma unroll
+          for (int k = 0; k < PX; k++)
+            if (k == i / GL) {
+              win[k] = arg;
+              least[k] = m;
+              beside[k] = bs;
+            }
+        }
+        __syncwarp();
+      }
+    };
+    if (plain) {
+#pragma unroll
+      for (int i = kSeg - 1; i >= 0; i--) {
+        L4 raw2;
+        unpack_cost(raw2, rawp[i * 32], pad);
+        line_step<GL, kBeyond>(B, bd, raw2, a.p2x2, a, first, last);
+        put(i, pi0 + step * i, true);
+        if (in) stage(i, pq + step * i);
+      }
+    } else {
+      int x = x0 + dx * (kSeg - 1), pi = pi0 + step * (kSeg - 1);
+      if ((unsigned)x >= (unsigned)W) x -= dx * W;
+#pragma unroll 1
+      for (int i = kSeg - 1; i >= 0; i--) {
+        // the line's last pixel, or a new line: the way back comes in at the side the diagonal left by
+        if (t0 + i == NS - 1 || (P == 1 && x == W - 1) || (P == 3 && x == 0)) set_zero(B, bd);
+        L4 raw2;
+        unpack_cost(raw2, rawp[i * 32], pad);
+        line_step<GL, kBeyond>(B, bd, raw2, a.p2x2, a, first, last);
+        put(i, pi, t0 + i < NS);
+        if (seg > 0 && in && t0 - kSeg + i < NS) stage(i, pq + step * i);
+        pi -= step;
+        x -= dx;
+        if ((unsigned)x >= (unsigned)W) x += dx * W;
+      }
+    }
+    cp_async_commit();
+    if (MODE == 2 && gl < kSeg) {
+#pragma unroll
+      for (int k = 0; k < PX; k++) {
+        const int i = gl + k * GL;
+        if (in && t0 + i < NS) {
+          pr.dl[pi0 + step * i] = win[k];
+          pr.disp[pi0 + step * i] = refine(win[k], pr.D, a.subpixel, (float)least[k], (float)(beside[k] & 0xffffu), (float)(beside[k] >> 16));
+        }
+      }
+    }
+    F = Fn;
+    fd = dup16(fdn);
+    pi0 = pq;
+    x0 -= dx * kSeg;
+    if ((unsigned)x0 >= (unsigned)W) x0 += dx * W;
+  }
+}
+
+// The pair walk of path P (its warps first) beside the forward walk of path NEXT; -1: none. A grid row a pair of images.
+template <int GL, int P, int MODE, int NEXT>
+__global__ void __launch_bounds__(64, 16) k_census_walk(const __grid_constant__ CensusLines a) {
+  constexpr int LPW = 32 / GL, PP = P < 0 ? 0 : P, PN = NEXT < 0 ? 0 : NEXT;
+  __shared__ uint4 s_sum[2][kSeg * 32];
+  __shared__ uint2 s_raw[2][kSeg * 32];
+  const int wib = threadIdx.x >> 5;
+  const CensusPair& pr = a.ps.p[blockIdx.y];
+  uint16_t* ckpt[2];
+  uint16_t* ckpt_min[2];
+  for (int k = 0; k < 2; k++) {
+    ckpt[k] = a.ckpt + (blockIdx.y * 2 + k) * a.states * a.n;
+    ckpt_min[k] = a.ckpt_min + (blockIdx.y * 2 + k) * a.states;
+  }
+  const int pair_blocks = P < 0 ? 0 : ((line_count(a, PP) + LPW - 1) / LPW + 1) / 2, block = blockIdx.x;
+  if (P >= 0 && block < pair_blocks) {
+    census_pair<GL, PP, MODE>(a, pr, block * 2 + wib, s_sum[wib], s_raw[wib], ckpt[PP & 1], ckpt_min[PP & 1]);
+  } else if (NEXT >= 0) {
+    census_forward<GL, PN>(a, pr, (block - pair_blocks) * 2 + wib, reinterpret_cast<uint2*>(s_sum[wib]), ckpt[PN & 1], ckpt_min[PN & 1]);
+  }
+}
+
+template <int GL, int P, int MODE, int NEXT>
+void run_census_walk(const CensusLines& a, int n, cudaStream_t s) {
+  constexpr int LPW = 32 / GL;
+  auto blocks_of = [&](int p) {
+    const int lines = p < 0 ? 0 : p == 0 ? a.H : p == 1 ? a.W + 1 : p == 2 ? a.W : a.W - 1;
+    return ((lines + LPW - 1) / LPW + 1) / 2;
+  };
+  k_census_walk<GL, P, MODE, NEXT><<<dim3(blocks_of(P) + blocks_of(NEXT), n), 64, 0, s>>>(a);
+}
+
+// The right image's first minimum over d of S(x + d, y, d), x + d < W (a warp per right-image pixel). OCTETS: the sums are in
+// the lines' order.
+template <int LPT, bool OCTETS>
 __global__ void __launch_bounds__(256) k_census_wta_right(const CensusPairs ps, int w, int h) {
   constexpr int Dp = 32 * LPT;
   const CensusPair& pr = ps.p[blockIdx.y];
@@ -269,7 +563,7 @@ __global__ void __launch_bounds__(256) k_census_wta_right(const CensusPairs ps, 
 #pragma unroll
   for (int i = 0; i < LPT; i++) {
     const int d = lane * LPT + i;
-    const uint32_t v = d < D && x + d < w ? __ldg(S + ((size_t)y * w + x + d) * Dp + d) : kBig;
+    const uint32_t v = d < D && x + d < w ? __ldg(S + ((size_t)y * w + x + d) * Dp + (OCTETS ? (d & ~7) + octet_pos(d & 7) : d)) : kBig;
     if (v < best) {
       best = v;
       arg = d;
@@ -316,20 +610,48 @@ __global__ void k_fuse(const float* const* __restrict__ disps, const float* __re
 
 template <int LPT>
 void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h, uint32_t P1, uint32_t P2, int subpixel, int lr,
-                  int max_diff, cudaStream_t s) {
+                  int max_diff, const CensusScratch& sc, cudaStream_t s) {
   const int npx = w * h;
+  constexpr int GL = 4 * LPT;
   k_hamming<LPT><<<dim3((unsigned)((npx + 7) / 8), n), 256, 0, s>>>(cl, ps, w, h);
-  static const int dirs[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {-1, -1}, {1, -1}, {-1, 1}};
-  for (int k = 0; k < 8; k++) {
-    const int dx = dirs[k][0], dy = dirs[k][1];
-    const int lines = (dy != 0 ? w : 0) + (dx != 0 ? h - (dy != 0 ? 1 : 0) : 0);
-    const dim3 grid((lines + 3) / 4, n);
-    if (k == 7) k_census_path<LPT, true><<<grid, 128, 0, s>>>(ps, w, h, dx, dy, P1, P2, 0, subpixel);
-    else k_census_path<LPT, false><<<grid, 128, 0, s>>>(ps, w, h, dx, dy, P1, P2, k == 0 ? 1 : 0, subpixel);
+  count_launches(1);
+  if (sc.ckpt) {
+    CensusLines a{};
+    a.W = w;
+    a.H = h;
+    a.n = 32 * LPT;
+    a.p1x2 = P1 * 0x10001u;
+    a.p2x2 = P2 * 0x10001u;
+    a.one = 1;
+    a.subpixel = subpixel;
+    a.keep = lr;
+    a.states = census_states(w, h);
+    a.ckpt = sc.ckpt;
+    a.ckpt_min = sc.ckpt_min;
+    for (int k0 = 0; k0 < n; k0 += sc.pairs) {
+      const int m = std::min(sc.pairs, n - k0);
+      for (int k = 0; k < m; k++) a.ps.p[k] = ps.p[k0 + k];
+      run_census_walk<GL, -1, 0, 0>(a, m, s);
+      run_census_walk<GL, 0, 0, 1>(a, m, s);
+      run_census_walk<GL, 1, 1, 2>(a, m, s);
+      run_census_walk<GL, 2, 1, 3>(a, m, s);
+      run_census_walk<GL, 3, 2, -1>(a, m, s);
+      count_launches(5);
+    }
+  } else {
+    static const int dirs[8][2] = {{1, 0}, {-1, 0}, {0, 1}, {0, -1}, {1, 1}, {-1, -1}, {1, -1}, {-1, 1}};
+    for (int k = 0; k < 8; k++) {
+      const int dx = dirs[k][0], dy = dirs[k][1];
+      const int lines = (dy != 0 ? w : 0) + (dx != 0 ? h - (dy != 0 ? 1 : 0) : 0);
+      const dim3 grid((lines + 3) / 4, n);
+      if (k == 7) k_census_path<LPT, true><<<grid, 128, 0, s>>>(ps, w, h, dx, dy, P1, P2, 0, subpixel);
+      else k_census_path<LPT, false><<<grid, 128, 0, s>>>(ps, w, h, dx, dy, P1, P2, k == 0 ? 1 : 0, subpixel);
+    }
+    count_launches(8);
   }
-  count_launches(9);
   if (lr) {
-    k_census_wta_right<LPT><<<dim3((npx + 7) / 8, n), 256, 0, s>>>(ps, w, h);
+    if (sc.ckpt) k_census_wta_right<LPT, true><<<dim3((npx + 7) / 8, n), 256, 0, s>>>(ps, w, h);
+    else k_census_wta_right<LPT, false><<<dim3((npx + 7) / 8, n), 256, 0, s>>>(ps, w, h);
     k_census_lr<<<dim3((npx + 255) / 256, n), 256, 0, s>>>(ps, w, h, max_diff);
     count_launches(2);
   }
@@ -337,10 +659,15 @@ void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h
 
 }  // namespace
 
+// The states of the longest walk of a pair: W + 1 lines or fewer of at most H + H / (W - 1) + 1 steps, or H lines of W.
+size_t census_states(int w, int h) {
+  return std::max((size_t)(w + 1) * ((h + h / (w - 1) + 1) / kSeg + 1), (size_t)h * (w / kSeg + 1));
+}
+bool census_lines_supported(int w) { return w >= kBatch; }
 int census_lpt(int D) { return D <= 32 ? 1 : D <= 64 ? 2 : D <= 128 ? 4 : D <= 256 ? 8 : 0; }
 
 void launch_census_batch(const uint8_t* ref, const uint8_t* const* others, int n, int w, int h, int stride, int bpp, uint32_t P1,
-                         uint32_t P2, int subpixel, int lr, int max_diff, uint64_t* cl, const CensusPairs& ps, cudaStream_t s) {
+                         uint32_t P2, int subpixel, int lr, int max_diff, uint64_t* cl, const CensusPairs& ps, const CensusScratch& sc, cudaStream_t s) {
   const dim3 b2(32, 8), g2((w + 31) / 32, (h + 7) / 8);
   k_census<<<g2, b2, 0, s>>>(ref, w, h, stride, bpp, cl);  // the reference's census, shared by every pair
   for (int k = 0; k < n; k++) k_census<<<g2, b2, 0, s>>>(others[k], w, h, stride, bpp, ps.p[k].cr);
@@ -353,10 +680,10 @@ void launch_census_batch(const uint8_t* ref, const uint8_t* const* others, int n
       if (census_lpt(ps.p[k].D) == lpt) grp.p[m++] = ps.p[k];
     if (m == 0) continue;
     switch (lpt) {
-      case 1: batch_stages<1>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, s); break;
-      case 2: batch_stages<2>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, s); break;
-      case 4: batch_stages<4>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, s); break;
-      default: batch_stages<8>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, s); break;
+      case 1: batch_stages<1>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, sc, s); break;
+      case 2: batch_stages<2>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, sc, s); break;
+      case 4: batch_stages<4>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, sc, s); break;
+      default: batch_stages<8>(cl, grp, m, w, h, P1, P2, subpixel, lr, max_diff, sc, s); break;
     }
   }
 }

@@ -117,11 +117,19 @@ struct CensusPair {
 struct CensusPairs {
   CensusPair p[kMaxFusePairs];
 };
+// Where the walks along lines keep their states: 2 x census_states for each of the pairs walked at once (ckpt null: one warp walks
+// a scanline instead, without kept states).
+struct CensusScratch {
+  uint16_t *ckpt, *ckpt_min;
+  int pairs;
+};
+bool census_lines_supported(int w);      // the widths that the lines take
+size_t census_states(int w, int h);      // kept states of a path: each of 32·census_lpt(D) values and a minimum, twice a pair
 // n pairs (<= kMaxFusePairs) of the reference image against others[k] (device pointers), all W x H; grey at byte 0 of
 // every bpp bytes, rows stride pixels apart; pair k's buffers are laid out with 32·census_lpt(D_k) values a pixel; cl:
 // the reference's census (W x H). One launch per stage covers every pair of the same lane width.
 void launch_census_batch(const uint8_t* ref, const uint8_t* const* others, int n, int w, int h, int stride, int bpp, uint32_t P1,
-                         uint32_t P2, int subpixel, int lr, int max_diff, uint64_t* cl, const CensusPairs& ps, cudaStream_t s);
+                         uint32_t P2, int subpixel, int lr, int max_diff, uint64_t* cl, const CensusPairs& ps, const CensusScratch& sc, cudaStream_t s);
 // disps: a device array of n device pointers to W x H disparity maps (n <= kMaxFusePairs); fb: n focal x baseline products.
 void launch_fuse(const float* const* disps, const float* fb, int n, int npx, float* out, cudaStream_t s);
 

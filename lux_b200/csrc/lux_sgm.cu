@@ -158,6 +158,15 @@ int alloc_t(lux_sgm_ctx* ctx, std::vector<DevBuf>& owner, size_t count, T** out)
   return rc;
 }
 
+// The same for memory that a call can do without: no error is set.
+template <class T>
+int alloc_quiet(lux_sgm_ctx* ctx, std::vector<DevBuf>& owner, size_t count, T** out) {
+  const std::string kept = ctx->last_error;
+  const int rc = alloc_t(ctx, owner, count, out);
+  if (rc) ctx->last_error = kept;
+  return rc;
+}
+
 // Reads and clears the device error word.
 int take_device_error(lux_sgm_ctx* ctx) {
   int e = 0;
@@ -1245,7 +1254,19 @@ int census_batch(lux_sgm_ctx* ctx, std::vector<DevBuf>& tmp, int n, const lux_im
     if (!rc) rc = alloc_t(ctx, tmp, npx, &pr.disp);
   }
   if (rc) return rc;
-  launch_census_batch(d_ref, d_oth.data(), n, w, h, w, 4, p1, p2, subpixel, lr, max_diff, cl, pairs, ctx->stream);
+  // The lines' kept states (a sixth of the pairs' own memory), for as many pairs at once as 2 GB hold: enough to fill the GPU.
+  // Where the memory or the context's budget does not have them, the scanlines are walked without.
+  CensusScratch sc{};
+  std::vector<DevBuf> states;
+  if (census_lines_supported(w)) {
+    size_t Dp = 0;
+    for (int k = 0; k < n; k++) Dp = std::max(Dp, 32 * (size_t)census_lpt(Ds[k]));
+    const size_t per = 2 * census_states(w, h);
+    sc.pairs = (int)std::min<size_t>(n, std::max<size_t>(1, ((size_t)2 << 30) / (per * (Dp + 1) * 2)));
+    if (alloc_quiet(ctx, states, per * sc.pairs * Dp, &sc.ckpt) || alloc_quiet(ctx, states, per * sc.pairs, &sc.ckpt_min)) sc.ckpt = nullptr;
+  }
+  launch_census_batch(d_ref, d_oth.data(), n, w, h, w, 4, p1, p2, subpixel, lr, max_diff, cl, pairs, sc, ctx->stream);
+  dev_free_all(ctx, states);
   CK(cudaGetLastError());
   return LUX_OK;
 }
