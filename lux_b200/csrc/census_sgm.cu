@@ -85,26 +85,43 @@ __global__ void k_census(const uint8_t* __restrict__ img, int w, int h, int stri
   out[(size_t)y * w + x] = v;
 }
 
-// C(x, y, d) = popcount(L(x, y) ^ R(x - d, y)), 62 where x - d < 0. A warp per pixel, lane j making disparities j, j + 32,
-// ...: each load instruction reads 32 neighbouring right-image words and each store writes 32 consecutive cost bytes.
+// C(x, y, d) = popcount(L(x, y) ^ R(x - d, y)), 62 where x - d < 0. A block takes kHamTile pixels of a row, a thread eight
+// disparities of a pixel at a time, stored as one word pair; the right image's words wait in shared memory, their halves apart
+// and a word skipped every eight, so that threads eight words apart meet no bank twice. Bound by the population counts (16 a
+// clock an SM): 2080x1560 D=128 in 273 us; a warp a pixel storing bytes took 418, this from global memory 769.
+constexpr int kHamTile = 64;
 template <int LPT>
-__global__ void __launch_bounds__(256) k_hamming(const uint64_t* __restrict__ cl, const CensusPairs ps, int w, int h) {
-  constexpr int Dp = 32 * LPT;
+__global__ void __launch_bounds__(256) k_hamming(const uint64_t* __restrict__ cl, const CensusPairs ps, int w, int h, int tiles) {
+  constexpr int Dp = 32 * LPT, GL = 4 * LPT, kWords = kHamTile + Dp - 1;  // GL: threads of a pixel
+  __shared__ uint32_t lo[kWords + kWords / 8 + 1], hi[kWords + kWords / 8 + 1];
   const CensusPair& pr = ps.p[blockIdx.y];  // one grid row per pair of the batch
-  const uint64_t* __restrict__ cr = pr.cr;
-  uint8_t* __restrict__ cost = pr.cost;
-  const int D = pr.D;
-  const int lane = threadIdx.x & 31;
-  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (p >= w * h) return;
-  const int y = p / w, x = p - y * w;
-  const uint64_t a = __ldg(cl + p);
-  const uint64_t* row = cr + (size_t)y * w;
-  uint8_t* out = cost + (size_t)p * Dp;
+  const int y = blockIdx.x / tiles, x0 = (blockIdx.x - y * tiles) * kHamTile, D = pr.D;
+  for (int i = threadIdx.x; i < kWords; i += 256) {  // word i: R(x0 - (Dp - 1) + i, y)
+    const int xr = x0 - (Dp - 1) + i;
+    const uint64_t v = xr >= 0 && xr < w ? __ldg(pr.cr + (size_t)y * w + xr) : 0;
+    lo[i + i / 8] = (uint32_t)v;
+    hi[i + i / 8] = (uint32_t)(v >> 32);
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < kHamTile * GL; t += 256) {
+    const int x = x0 + t / GL, d0 = (t % GL) * 8;
+    if (x >= w) break;
+    const size_t p = (size_t)y * w + x;
+    const uint64_t a = __ldg(cl + p);
+    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32);
+    const int r = t / GL + Dp - 1 - d0, live = min(D - d0, x - d0 + 1);  // the word of d0; how many of the disparities count
+    uint32_t c[8];
 #pragma unroll
-  for (int k = 0; k < LPT; k++) {
-    const int d = lane + 32 * k;
-    out[d] = (uint8_t)(d < D && x - d >= 0 ? __popcll(a ^ __ldg(row + x - d)) : kInvalidCost);
+    for (int i = 0; i < 8; i++) {
+      const int j = r - i + (r - i) / 8;
+      c[i] = __popc(al ^ lo[j]) + __popc(ah ^ hi[j]);
+    }
+    if (live < 8) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) c[i] = i < live ? c[i] : kInvalidCost;
+    }
+    reinterpret_cast<uint2*>(pr.cost + p * Dp)[t % GL] =
+        make_uint2(c[0] | c[1] << 8 | c[2] << 16 | c[3] << 24, c[4] | c[5] << 8 | c[6] << 16 | c[7] << 24);
   }
 }
 
@@ -268,7 +285,7 @@ __global__ void __launch_bounds__(128) k_census_path(const CensusPairs ps, int w
 // above m + P2 also as neighbours. Their sums may wrap: the high half of a pair never carries into a true one (plane p + 4
 // is past D where plane p is), and the winner-take-all takes them as 0xffff (eight true L sum up to 65528 at most).
 // The eight walks of one disparity a lane, one warp a line and one pixel of prefetch took 10.4 ms at 2080x1560 D=128 (each
-// was bound by its steps' latency, at 1.2 TB/s); these take 3.5 ms.
+// was bound by its steps' latency, at 1.2 TB/s); these take 3.0 ms.
 constexpr uint32_t kBeyond = 0x40004000u;
 
 struct CensusLines {
@@ -546,32 +563,43 @@ void run_census_walk(const CensusLines& a, int n, cudaStream_t s) {
   k_census_walk<GL, P, MODE, NEXT><<<dim3(blocks_of(P) + blocks_of(NEXT), n), 64, 0, s>>>(a);
 }
 
-// The right image's first minimum over d of S(x + d, y, d), x + d < W (a warp per right-image pixel). OCTETS: the sums are in
-// the lines' order.
+// The right image's first minimum over d of S(x + d, y, d), x + d < W. A block takes kRight right pixels of a row, a thread each,
+// sixteen disparities at a time: their sums of the kRight + 15 left pixels they meet (a sector of each) go through shared
+// memory, nine words apart so that a warp's diagonal reads meet no bank twice. Bound by HBM: 2080x1560 D=128 in 231 us; a
+// warp a right pixel, reading its sums where they lay, took 580. OCTETS: the sums are in the lines' order.
+constexpr int kRight = 128;
 template <int LPT, bool OCTETS>
-__global__ void __launch_bounds__(256) k_census_wta_right(const CensusPairs ps, int w, int h) {
-  constexpr int Dp = 32 * LPT;
+__global__ void __launch_bounds__(kRight) k_census_wta_right(const CensusPairs ps, int w, int h, int tiles) {
+  constexpr int Dp = 32 * LPT, kWide = kRight + 15;
+  __shared__ uint32_t sums[2][kWide * 9];
   const CensusPair& pr = ps.p[blockIdx.y];
-  const uint16_t* __restrict__ S = pr.S;
-  int* __restrict__ dr = pr.dr;
-  const int D = pr.D;
-  const int lane = threadIdx.x & 31;
-  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (p >= w * h) return;
-  const int y = p / w, x = p - y * w;
-  uint32_t best = kBig, arg = kBig;
+  const int y = blockIdx.x / tiles, x0 = (blockIdx.x - y * tiles) * kRight, x = x0 + threadIdx.x;
+  const uint16_t* row = pr.S + (size_t)y * w * Dp;
+  uint32_t best = ~0u;  // the sum, then the disparity
+  const int chunks = min((pr.D + 15) / 16, (w - x0 + 15) / 16);
+  for (int c = 0; c < chunks; c++) {
+    uint32_t* buf = sums[c & 1];  // (a thread is at most one chunk ahead of another)
+    const int xa = x0 + c * 16;
+    for (int i = threadIdx.x; i < kWide * 2; i += kRight) {
+      const int px = i >> 1, hf = i & 1;
+      if (xa + px >= w) break;
+      const uint4 v = __ldcs(reinterpret_cast<const uint4*>(row + (size_t)(xa + px) * Dp + c * 16) + hf);
+      uint32_t* q = buf + px * 9 + hf * 4;
+      q[0] = v.x;
+      q[1] = v.y;
+      q[2] = v.z;
+      q[3] = v.w;
+    }
+    __syncthreads();
+    const uint16_t* mine = reinterpret_cast<const uint16_t*>(buf + threadIdx.x * 9);
 #pragma unroll
-  for (int i = 0; i < LPT; i++) {
-    const int d = lane * LPT + i;
-    const uint32_t v = d < D && x + d < w ? __ldg(S + ((size_t)y * w + x + d) * Dp + (OCTETS ? (d & ~7) + octet_pos(d & 7) : d)) : kBig;
-    if (v < best) {
-      best = v;
-      arg = d;
+    for (int i = 0; i < 16; i++) {
+      const int d = c * 16 + i;
+      const uint32_t v = mine[i * 18 + (OCTETS ? (i & 8) + octet_pos(i & 7) : i)];
+      if (d < pr.D && x + d < w) best = min(best, v << 8 | (uint32_t)d);
     }
   }
-  const uint32_t m = __reduce_min_sync(0xffffffffu, best);
-  const uint32_t d = __reduce_min_sync(0xffffffffu, best == m ? arg : kBig);
-  if (lane == 0) dr[p] = (int)d;
+  if (x < w) pr.dr[(size_t)y * w + x] = (int)(best & 0xffu);
 }
 
 // Left/right consistency: a pixel keeps its disparity when |d(x) - d_R(x - d(x))| <= max_diff, else -1.
@@ -613,7 +641,8 @@ void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h
                   int max_diff, const CensusScratch& sc, cudaStream_t s) {
   const int npx = w * h;
   constexpr int GL = 4 * LPT;
-  k_hamming<LPT><<<dim3((unsigned)((npx + 7) / 8), n), 256, 0, s>>>(cl, ps, w, h);
+  const int tiles_h = (w + kHamTile - 1) / kHamTile;
+  k_hamming<LPT><<<dim3((unsigned)tiles_h * h, n), 256, 0, s>>>(cl, ps, w, h, tiles_h);
   count_launches(1);
   if (sc.ckpt) {
     CensusLines a{};
@@ -650,8 +679,10 @@ void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h
     count_launches(8);
   }
   if (lr) {
-    if (sc.ckpt) k_census_wta_right<LPT, true><<<dim3((npx + 7) / 8, n), 256, 0, s>>>(ps, w, h);
-    else k_census_wta_right<LPT, false><<<dim3((npx + 7) / 8, n), 256, 0, s>>>(ps, w, h);
+    const int tiles = (w + kRight - 1) / kRight;
+    const dim3 right((unsigned)tiles * h, n);
+    if (sc.ckpt) k_census_wta_right<LPT, true><<<right, kRight, 0, s>>>(ps, w, h, tiles);
+    else k_census_wta_right<LPT, false><<<right, kRight, 0, s>>>(ps, w, h, tiles);
     k_census_lr<<<dim3((npx + 255) / 256, n), 256, 0, s>>>(ps, w, h, max_diff);
     count_launches(2);
   }
