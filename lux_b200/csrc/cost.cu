@@ -9,10 +9,11 @@
 // Half-pixel phases: the resampled block value at (x, y) with fractions (hx, hy) is pavgb over rows first, then over
 // columns, of the 2x2 neighbourhood at (x, y) (:248-253); it depends on (x, y, hx, hy) only, so k_phase_* writes the four
 // phase images of every other camera once per layer and a plane's 3x3 block is three row loads with no averaging:
-//   grey camera (weights {12240, 0, 0, 0}, only Y contributes): per pixel and phase the Y bytes of columns x, x+1, x+2
-//     as u16 pairs {x | x+2 << 16, x+1}, so a block row is one 8-byte load; |t - r| capped at 2 in u16x2 lanes;
+//   grey camera (weights {12240, 0, 0, 0}, only Y contributes): per pixel and phase the Y bytes of columns x, x+1, x+2 in
+//     a word, so a block row is one 4-byte load and its differences one instruction, capped at 2 in u16x2 lanes;
 //   colour camera: the RGBA word per pixel and phase; even bytes (Y, V) and odd bytes (U, A) as u16x2 lanes.
 // Both are exact restatements of the reference's byte-lane sums (each channel sum is at most 9·6).
+#include <algorithm>
 #include <climits>
 
 #include "common.cuh"
@@ -30,7 +31,6 @@ LUX_DEV uint32_t vmax2c(uint32_t a, uint32_t b) {
   asm("max.u16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
-LUX_DEV uint32_t absdiff2(uint32_t a, uint32_t b) { return vmax2c(a, b) - vmin2c(a, b); }  // per u16 lane, no borrow
 LUX_DEV int avg_u8(int a, int b) { return (a + b + 1) >> 1; }                 // pavgb on one byte
 
 // The phase-h value (h = 2·hy + hx) of byte channel `ch` at (x, y): rows averaged first, then columns. Only positions
@@ -46,16 +46,22 @@ LUX_DEV int phase_byte(const uint8_t* img, int iw, int ih, int x, int y, int h, 
   return (h & 1) ? avg_u8(a, b) : a;
 }
 
-// Grey: out[h][y][x] = the Y bytes of phase h at columns x, x+1, x+2 as u16 pairs: {x | x+2 << 16, x+1}.
-__global__ void k_phase_grey(const uint8_t* __restrict__ img, int iw, int ih, uint2* __restrict__ out) {
+// The two layouts without shared columns: half-pixel position (u, v) = (2x + hx, 2y + hy) at word v·2iw + u, so that a plane's
+// block starts one multiply-add away and planes half a pixel apart share their lines; a block's rows are 4iw words apart.
+// Grey: the Y bytes of phase 2·hy + hx at columns x, x+1, x+2, low byte first.
+__global__ void k_phase_grey(const uint8_t* __restrict__ img, int iw, int ih, uint32_t* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= iw) return;
+  uint32_t v[4];
 #pragma unroll
   for (int h = 0; h < 4; h++) {
     const uint32_t p0 = phase_byte(img, iw, ih, x, y, h, 0), p1 = phase_byte(img, iw, ih, min(x + 1, iw - 1), y, h, 0),
                    p2 = phase_byte(img, iw, ih, min(x + 2, iw - 1), y, h, 0);
-    out[((size_t)h * ih + y) * iw + x] = make_uint2(p0 | (p2 << 16), p1);
+    v[h] = p0 | p1 << 8 | p2 << 16;
   }
+  uint2* o = reinterpret_cast<uint2*>(out) + (size_t)y * 2 * iw + x;
+  o[0] = make_uint2(v[0], v[1]);
+  o[iw] = make_uint2(v[2], v[3]);
 }
 // Grey, vertical triples (the shared-column axis kernel): out[h][y][x] = the Y bytes of phase h at rows y, y+1, y+2 of
 // column x as u16 pairs: {y | y+2 << 16, y+1}.
@@ -69,65 +75,73 @@ __global__ void k_phase_grey_v(const uint8_t* __restrict__ img, int iw, int ih, 
     out[((size_t)h * ih + y) * iw + x] = make_uint2(p0 | (p2 << 16), p1);
   }
 }
-// Colour: out[h][y][x] = the RGBA word of phase h.
+// Colour: the RGBA word of the phase.
 __global__ void k_phase_colour(const uint8_t* __restrict__ img, int iw, int ih, uint32_t* __restrict__ out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= iw) return;
+  uint32_t v[4];
 #pragma unroll
   for (int h = 0; h < 4; h++) {
-    uint32_t v = 0;
+    v[h] = 0;
 #pragma unroll
-    for (int ch = 0; ch < 4; ch++) v |= (uint32_t)phase_byte(img, iw, ih, x, y, h, ch) << (8 * ch);
-    out[((size_t)h * ih + y) * iw + x] = v;
+    for (int ch = 0; ch < 4; ch++) v[h] |= (uint32_t)phase_byte(img, iw, ih, x, y, h, ch) << (8 * ch);
   }
+  uint2* o = reinterpret_cast<uint2*>(out) + (size_t)y * 2 * iw + x;
+  o[0] = make_uint2(v[0], v[1]);
+  o[iw] = make_uint2(v[2], v[3]);
 }
 
-// Grey block: S0 = Σ min(|t - r|, 2) over the 3x3 Y block. Row r of the target is one 8-byte load {t0 | t2 << 16, t1}.
-// In each u16 lane max(t + (256 - r), (256 + r) - t) = 256 + |t - r|, so min(., 258) - 256 is the capped difference
-// with two adds and two min/max instead of three min/max and a subtract (the 256s are removed once, at the end); the
-// unused upper lane of the odd word is capped at 256 (a zero term).
+// Grey block: S0 = Σ min(|t - r|, 2) over the 3x3 Y block, a row's three bytes in a word (the top bytes are equal: zero).
 struct GreyRef {
-  uint32_t ea[3], eb[3], oa[3], ob[3];  // per row: 256 - r and 256 + r for the lanes {r0, r2} and {r1, 0}
+  uint32_t r[3];
 };
-LUX_DEV GreyRef grey_ref(const uint32_t (&ge)[3], const uint32_t (&go)[3]) {
+LUX_DEV GreyRef grey_ref(const uint32_t (&rb)[3][3]) {
   GreyRef g;
 #pragma unroll
-  for (int r = 0; r < 3; r++) {
-    g.ea[r] = 0x01000100u - ge[r];
-    g.eb[r] = 0x01000100u + ge[r];
-    g.oa[r] = 0x01000100u - go[r];
-    g.ob[r] = 0x01000100u + go[r];
-  }
+  for (int r = 0; r < 3; r++) g.r[r] = (rb[r][0] & 0xffu) | (rb[r][1] & 0xffu) << 8 | (rb[r][2] & 0xffu) << 16;
   return g;
 }
-LUX_DEV int grey_cost(const uint2* __restrict__ q, int iw, const GreyRef& g) {
-  uint32_t s = 0;
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    const uint2 t = __ldg(q + (size_t)r * iw);
-    s += vmin2c(vmax2c(t.x + g.ea[r], g.eb[r] - t.x), 0x01020102u) + vmin2c(vmax2c(t.y + g.oa[r], g.ob[r] - t.y), 0x01000102u);
-  }
-  const int S0 = (int)((s & 0xffffu) + (s >> 16)) - 12 * 256;
-  return (S0 * 12240 + 16) >> 5;
+LUX_DEV int grey_sum(const uint32_t (&t)[3], const GreyRef& g) {
+  const uint32_t v0 = __vabsdiffu4(t[0], g.r[0]), v1 = __vabsdiffu4(t[1], g.r[1]), v2 = __vabsdiffu4(t[2], g.r[2]);
+  const uint32_t two = 0x00020002u, m = 0x00ff00ffu;
+  const uint32_t s = vmin2c(v0 & m, two) + vmin2c(v1 & m, two) + vmin2c(v2 & m, two) + vmin2c(__byte_perm(v0, v1, 0x3531), two) +
+                     vmin2c(__byte_perm(v2, 0, 0x4441), two);  // (byte 3 of a difference is zero)
+  return (int)((s & 0xffffu) + (s >> 16));
+}
+LUX_DEV int grey_weighted(int s0) { return (s0 * 12240 + 16) >> 5; }
+LUX_DEV int grey_cost(const uint32_t* __restrict__ q, int iw, const GreyRef& g) {
+  const uint32_t t[3] = {__ldg(q), __ldg(q + 4 * (size_t)iw), __ldg(q + 8 * (size_t)iw)};
+  return grey_weighted(grey_sum(t, g));
 }
 
-// Colour block: even bytes (Y, V) and odd bytes (U, A) as u16 pairs, caps {Y:2, V:6} and {U:6, A:0}.
-LUX_DEV int colour_cost(const uint32_t* __restrict__ q, int iw, const uint32_t (&re)[3][3], const uint32_t (&ro)[3][3],
-                        const uint16_t (&wq)[4]) {
-  const uint32_t capE = 0x00060002u, capO = 0x00000006u;
-  uint32_t se = 0, so = 0;
+// The reference 3x3 block, rows and columns clamped to the image.
+LUX_DEV void ref_block(const CostArgs& a, int xImg, int yImg, uint32_t (&rb)[3][3]) {
 #pragma unroll
   for (int r = 0; r < 3; r++) {
+    const int yy = min(max(yImg + r - 1, 0), a.rh - 1);
 #pragma unroll
-    for (int p = 0; p < 3; p++) {
-      const uint32_t w = __ldg(q + (size_t)r * iw + p);
-      se += vmin2c(absdiff2(w & 0x00ff00ffu, re[r][p]), capE);
-      so += vmin2c(absdiff2((w >> 8) & 0x00ff00ffu, ro[r][p]), capO);
-    }
+    for (int c = 0; c < 3; c++)
+      rb[r][c] = __ldg(reinterpret_cast<const uint32_t*>(a.ref) + (size_t)yy * a.rw + min(max(xImg + c - 1, 0), a.rw - 1));
   }
-  const int S0 = se & 0xffff, S2 = se >> 16, S1 = so & 0xffff, S3 = so >> 16;
-  const int cY = (S0 * wq[0] + 16) >> 5, cU = (S1 * wq[1] + 16) >> 5, cV = (S2 * wq[2] + 16) >> 5, cA = (S3 * wq[3] + 16) >> 5;
-  return (cY + cU) + (cV + cA);  // at most 6885: MathF.Min(…, 65535) and the float round trip change nothing
+}
+
+// Colour block: the four bytes' differences at once, then {Y, V} of a pixel and {U, U} of two as u16 pairs, capped at {2, 6}
+// and 6. A's cap is 0, so its sum is, and (0·w + 16) >> 5 adds nothing.
+LUX_DEV int colour_cost(const uint32_t* __restrict__ q, int iw, const uint32_t (&rb)[3][3], const uint16_t (&wq)[4]) {
+  uint32_t v[9], se = 0, so = 0;
+#pragma unroll
+  for (int i = 0; i < 9; i++) v[i] = __ldg(q + (size_t)(i / 3) * 4 * iw + 2 * (i % 3));
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    v[i] = __vabsdiffu4(v[i], rb[i / 3][i % 3]);
+    se += vmin2c(v[i] & 0x00ff00ffu, 0x00060002u);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) so += vmin2c(__byte_perm(v[i], v[i + 1], 0x5511) & 0x00ff00ffu, 0x00060006u);
+  so += min((v[8] >> 8) & 0xffu, 6u);
+  const int S0 = se & 0xffff, S2 = se >> 16, S1 = (so & 0xffff) + (so >> 16);
+  const int cY = (S0 * wq[0] + 16) >> 5, cU = (S1 * wq[1] + 16) >> 5, cV = (S2 * wq[2] + 16) >> 5;
+  return cY + cU + cV;  // at most 6885: MathF.Min(…, 65535) and the float round trip change nothing
 }
 
 template <bool GREY>
@@ -139,7 +153,6 @@ __global__ void __launch_bounds__(256) k_cost(const CostArgs a, const LayerGeom 
   const int npx = g.W * g.H;
   const int n = g.n_planes;
   const int half = (a.scale + (a.scale >> 31)) >> 1;
-  const uint32_t* ref = reinterpret_cast<const uint32_t*>(a.ref);
   for (int pi = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; pi < npx; pi += nwarps) {
     if (g.skip[pi]) {  // skipped pixels aggregate raw 0 and 255 past their count (DenseStereoSgm.cs:242)
       uint8_t* out = raw + g.off[pi];
@@ -155,23 +168,9 @@ __global__ void __launch_bounds__(256) k_cost(const CostArgs a, const LayerGeom 
       if (lane == 0) atomicCAS(err, 0, 7);
       continue;
     }
-    // the reference 3x3 block, rows/columns clamped to the image
-    uint32_t ge[3], go[3], re[3][3], ro[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      const int yy = min(max(yImg + r - 1, 0), a.rh - 1);
-      uint32_t yb[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const uint32_t w = __ldg(ref + (size_t)yy * a.rw + min(max(xImg + c - 1, 0), a.rw - 1));
-        yb[c] = w & 0xffu;
-        re[r][c] = w & 0x00ff00ffu;
-        ro[r][c] = (w >> 8) & 0x00ff00ffu;
-      }
-      ge[r] = yb[0] | (yb[2] << 16);
-      go[r] = yb[1];
-    }
-    const GreyRef gr = grey_ref(ge, go);
+    uint32_t rb[3][3];
+    ref_block(a, xImg, yImg, rb);
+    const GreyRef gr = grey_ref(rb);
     const float xf = (float)xImg, yf = (float)yImg;
     for (int c0 = 0; c0 < count; c0 += 32) {
       const int d = c0 + lane;
@@ -199,16 +198,16 @@ __global__ void __launch_bounds__(256) k_cost(const CostArgs a, const LayerGeom 
         // (int)(2f) gives the integer part (>> 1) and the half-pixel bit (& 1) wherever the position can be in the rect
         // (f >= 1); elsewhere both forms fall outside it
         const int tx = f2i(__fadd_rn(fx, fx)), ty = f2i(__fadd_rn(fy, fy));
-        const int ix = tx >> 1, iy = ty >> 1, h = ((ty & 1) << 1) | (tx & 1);
+        const int ix = tx >> 1, iy = ty >> 1;
         bool inb = valid && !(ix < x0 || ix >= x1 || iy < y0 || iy >= y1);
         if (d == 0 && !inb) {  // the scalar fallback of the reference would read out of the image
           atomicCAS(err, 0, 7);
         }
         int costK = 0;
         if (inb) {
-          const size_t qi = ((size_t)h * ih + (iy - 1)) * iw + (ix - 1);
-          if (GREY) costK = grey_cost(reinterpret_cast<const uint2*>(a.phase[k]) + qi, iw, gr);
-          else costK = colour_cost(a.phase[k] + qi, iw, re, ro, a.wq[k]);
+          const size_t qi = (size_t)(ty - 2) * (2 * iw) + (tx - 2);
+          if (GREY) costK = grey_cost(a.phase[k] + qi, iw, gr);
+          else costK = colour_cost(a.phase[k] + qi, iw, rb, a.wq[k]);
         }
         const uint32_t m = __ballot_sync(0xffffffffu, inb);
         const uint32_t below = m & ((1u << lane) - 1u);
@@ -228,94 +227,135 @@ __global__ void __launch_bounds__(256) k_cost(const CostArgs a, const LayerGeom 
   }
 }
 
+// 1/b rounded to nearest for 2^-125 <= |b| < 2^125, as __frcp_rn without its range checks and branch: one step of Markstein's
+// correction (IBM J. Res. Dev. 34(1), 1990) from an approximation within an ulp. Compared with __frcp_rn over every mantissa.
+LUX_DEV float rcp_mid(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return __fmaf_rn(__fmaf_rn(-b, r, 1.0f), r, r);
+}
+
 // Uniform layers (every pixel searches planes [0, n), cap n, n % 8 == 0; 1 to 15 other cameras): lanes over 32
-// neighbouring pixels of a row,
-// each lane walking its pixel's planes in order like the reference's loop, so the last computed cost of a camera
-// (:273-274) is a register, the plane terms are the same for the whole warp, and the camera constants stay in
-// registers. Eight planes of u8 costs go out per 8-byte store. Skipped pixels get raw 0 (DenseStereoSgm.cs:242).
-template <bool GREY, int NK>
-__global__ void __launch_bounds__(256) k_cost_rows(const CostArgs a, const LayerGeom g, const float4* __restrict__ zt,
+// neighbouring pixels of a row, each walking its pixel's planes in order like the reference's loop. Eight planes at a time
+// go through camera after camera: the camera's constants, its last computed cost (:273-274, kept in shared memory between
+// the eights) and the lines of its phase images are then in hand for eight planes, and eight costs go out in one store. Four
+// positions are projected and their blocks loaded together, unless no lane of the warp hits the camera's rect with any of
+// them. Bound by issue (57 instructions a camera and plane): ten grey cameras of 2080x1560 D=176 11.2 ms; with the cameras
+// inside the plane loop, and u16 pairs of twice the bytes, it took 22.7 (95 instructions, an eighth of the sectors from L1).
+// Skipped pixels get raw 0 (DenseStereoSgm.cs:242).
+constexpr int kRowsThreads = 128;
+template <bool GREY>
+__global__ void __launch_bounds__(kRowsThreads) k_cost_rows(const __grid_constant__ CostArgs a, const LayerGeom g, const float4* __restrict__ zt,
                                                    uint8_t* __restrict__ raw, int* err) {
+  __shared__ uint16_t s_last[kMaxCams][kRowsThreads];
   const int lane = threadIdx.x & 31;
   const int tiles_x = (g.W + 31) >> 5;
   const int ntiles = tiles_x * g.H;
   const int n = g.n_planes;
   const int half = (a.scale + (a.scale >> 31)) >> 1;
-  const uint32_t* ref = reinterpret_cast<const uint32_t*>(a.ref);
-  // NK cameras exactly (NK <= 4), or up to NK with a.n_others of them; the camera loops are unrolled, so the camera
-  // constants are kernel-argument operands
-  const int nk = NK <= 4 ? NK : a.n_others;
-  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += (gridDim.x * blockDim.x) >> 5) {
-    const int y = t / tiles_x, x = ((t - y * tiles_x) << 5) + lane;
-    if (x >= g.W) continue;
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t < ntiles) {
+    const int y = t / tiles_x, xr = ((t - y * tiles_x) << 5) + lane, x = min(xr, g.W - 1);
     const size_t pi = (size_t)y * g.W + x;
     uint8_t* out = raw + pi * n;
-    if (g.skip[pi]) {
+    const bool skipped = g.skip[pi] != 0, live = xr < g.W && !skipped;
+    if (xr < g.W && skipped)
       for (int d = 0; d < n; d += 8) *reinterpret_cast<uint2*>(out + d) = make_uint2(0u, 0u);
-      continue;
-    }
+    if (!__any_sync(0xffffffffu, live)) return;
     const int xImg = min(a.scale * x + half, a.rw - 1), yImg = min(a.scale * y + half, a.rh - 1);
-    uint32_t ge[3], go[3], re[3][3], ro[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; r++) {  // the reference 3x3 block, rows/columns clamped to the image
-      const int yy = min(max(yImg + r - 1, 0), a.rh - 1);
-      uint32_t yb[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const uint32_t w = __ldg(ref + (size_t)yy * a.rw + min(max(xImg + c - 1, 0), a.rw - 1));
-        yb[c] = w & 0xffu;
-        re[r][c] = w & 0x00ff00ffu;
-        ro[r][c] = (w >> 8) & 0x00ff00ffu;
-      }
-      ge[r] = yb[0] | (yb[2] << 16);
-      go[r] = yb[1];
-    }
-    const GreyRef gr = grey_ref(ge, go);
+    uint32_t rb[3][3];
+    ref_block(a, xImg, yImg, rb);
+    const GreyRef gr = grey_ref(rb);
     const float xf = (float)xImg, yf = (float)yImg;
-    int last[NK];
+    for (int d0 = 0; d0 < n; d0 += 8) {
+      float xz[8], yz[8];
+      uint32_t acc[8];
 #pragma unroll
-    for (int k = 0; k < NK; k++) last[k] = 0;
-    uint32_t pk0 = 0, pk1 = 0;
-    for (int d = 0; d < n; d++) {
-      const float z = __ldg(g.planes + d);
-      const float xz = __fmul_rn(xf, z), yz = __fmul_rn(yf, z);
-      uint32_t acc = 0;
-#pragma unroll
-      for (int k = 0; k < NK; k++) {
-        if (k >= nk) break;
+      for (int j = 0; j < 8; j++) {
+        const float z = __ldg(g.planes + d0 + j);
+        xz[j] = __fmul_rn(xf, z);
+        yz[j] = __fmul_rn(yf, z);
+        acc[j] = 0;
+      }
+#pragma unroll 1
+      for (int k = 0; k < a.n_others; k++) {
         const float* Wm = a.warp[k];
-        const int iwk = a.ow[k], ihk = a.oh[k];
-        const float4 zk = __ldg(zt + (size_t)k * n + d);
-        const float px = __fadd_rn(__fadd_rn(zk.x, __fmul_rn(xz, Wm[0])), __fmul_rn(yz, Wm[4]));
-        const float py = __fadd_rn(__fadd_rn(zk.y, __fmul_rn(xz, Wm[1])), __fmul_rn(yz, Wm[5]));
-        const float pz = __fadd_rn(__fadd_rn(zk.z, __fmul_rn(xz, Wm[2])), __fmul_rn(yz, Wm[6]));
-        const float inv = __frcp_rn(pz);
-        float fx = __fadd_rn(__fmul_rn(px, inv), 0.25f), fy = __fadd_rn(__fmul_rn(py, inv), 0.25f);
-        const int x1 = iwk - 2, y1 = ihk - 2;
-        if (d == 0) {  // the first plane is clamped into the rect (:263-269)
-          fx = cs_minf(cs_maxf(fx, 1.0f), (float)(x1 - 1));
-          fy = cs_minf(cs_maxf(fy, 1.0f), (float)(y1 - 1));
+        const float w0 = Wm[0], w1 = Wm[1], w2 = Wm[2], w4 = Wm[4], w5 = Wm[5], w6 = Wm[6];
+        const int iw = a.ow[k], ih = a.oh[k];
+        const unsigned wide = (unsigned)max(2 * iw - 6, 0), high = (unsigned)max(2 * ih - 6, 0), pitch = 2 * (unsigned)iw;  // in half pixels
+        const uint32_t* phase = a.phase[k];
+        const float4* zk = zt + (size_t)k * n + d0;
+        int last = d0 > 0 ? s_last[k][threadIdx.x] : 0;
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+          float px[4], py[4], pz[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const float4 zj = __ldg(zk + q + j);
+            px[j] = __fadd_rn(__fadd_rn(zj.x, __fmul_rn(xz[q + j], w0)), __fmul_rn(yz[q + j], w4));
+            py[j] = __fadd_rn(__fadd_rn(zj.y, __fmul_rn(xz[q + j], w1)), __fmul_rn(yz[q + j], w5));
+            pz[j] = __fadd_rn(__fadd_rn(zj.z, __fmul_rn(xz[q + j], w2)), __fmul_rn(yz[q + j], w6));
+          }
+          float inv[4];
+          const float big = fmaxf(fmaxf(fabsf(pz[0]), fabsf(pz[1])), fmaxf(fabsf(pz[2]), fabsf(pz[3])));
+          const float small = fminf(fminf(fabsf(pz[0]), fabsf(pz[1])), fminf(fabsf(pz[2]), fabsf(pz[3])));
+          if (big < 0x1p125f && small >= 0x1p-125f) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) inv[j] = rcp_mid(pz[j]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) inv[j] = __frcp_rn(pz[j]);
+          }
+          int at[4];  // where the block starts in the phase images, -1 outside the rect
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            float fx = __fadd_rn(__fmul_rn(px[j], inv[j]), 0.25f), fy = __fadd_rn(__fmul_rn(py[j], inv[j]), 0.25f);
+            if (q + j == 0 && d0 == 0) {  // the first plane is clamped into the rect (:263-269)
+              fx = cs_minf(cs_maxf(fx, 1.0f), (float)(iw - 3));
+              fy = cs_minf(cs_maxf(fy, 1.0f), (float)(ih - 3));
+            }
+            // (int)(2f) - 2, the half-pixel position of the block's first row and column: the low bits of 2f + 1.5·2^23 rounded
+            // toward zero wherever the position can be in the rect, and past every rect for all other floats and NaN
+            const unsigned u = __float_as_uint(__fmaf_rz(fx, 2.0f, 12582912.0f)) - 0x4b400002u, v = __float_as_uint(__fmaf_rz(fy, 2.0f, 12582912.0f)) - 0x4b400002u;
+            const bool in = u < wide && v < high;
+            at[j] = in ? (int)(v * pitch + u) : -1;
+            // the scalar fallback of the reference would read out of the image
+            if (q + j == 0 && d0 == 0 && !in && live) atomicCAS(err, 0, 7);
+          }
+          if (!__any_sync(0xffffffffu, (at[0] & at[1] & at[2] & at[3]) >= 0)) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[q + j] += (uint32_t)last;
+            continue;
+          }
+          if (GREY) {
+            uint32_t w[4][3];
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const uint32_t* b = phase + max(at[j], 0);
+#pragma unroll
+              for (int r = 0; r < 3; r++) w[j][r] = __ldg(b + r * 2 * pitch);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const int c = grey_weighted(grey_sum(w[j], gr));
+              last = at[j] >= 0 ? c : last;
+              acc[q + j] += (uint32_t)last;
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              if (at[j] >= 0) last = colour_cost(phase + at[j], iw, rb, a.wq[k]);
+              acc[q + j] += (uint32_t)last;
+            }
+          }
         }
-        const int tx = f2i(__fadd_rn(fx, fx)), ty = f2i(__fadd_rn(fy, fy));
-        const int ix = tx >> 1, iy = ty >> 1;
-        if (ix >= 1 && ix < x1 && iy >= 1 && iy < y1) {
-          const int h = ((ty & 1) << 1) | (tx & 1);
-          const size_t qi = ((size_t)h * ihk + (iy - 1)) * iwk + (ix - 1);
-          last[k] = GREY ? grey_cost(reinterpret_cast<const uint2*>(a.phase[k]) + qi, iwk, gr)
-                         : colour_cost(a.phase[k] + qi, iwk, re, ro, a.wq[k]);
-        } else if (d == 0) {  // the scalar fallback of the reference would read out of the image
-          atomicCAS(err, 0, 7);
-        }
-        acc += (uint32_t)last[k];
+        s_last[k][threadIdx.x] = (uint16_t)last;
       }
-      const uint32_t b = (uint32_t)f2i(__fmul_rn((float)(acc & 0xffffu), a.norm)) & 0xffu;  // Normalise (:378-379)
-      const int sh = (d & 3) * 8;
-      if (d & 4) pk1 |= b << sh;
-      else pk0 |= b << sh;
-      if ((d & 7) == 7) {
-        *reinterpret_cast<uint2*>(out + (d - 7)) = make_uint2(pk0, pk1);
-        pk0 = pk1 = 0;
-      }
+      uint32_t pk[2] = {0, 0};
+#pragma unroll
+      for (int j = 0; j < 8; j++)  // Normalise (:378-379)
+        pk[j >> 2] |= ((uint32_t)f2i(__fmul_rn((float)(acc[j] & 0xffffu), a.norm)) & 0xffu) << (8 * (j & 3));
+      if (live) *reinterpret_cast<uint2*>(out + d0) = make_uint2(pk[0], pk[1]);
     }
   }
 }
@@ -336,12 +376,10 @@ __global__ void __launch_bounds__(256) k_cost_axis(const CostArgs a, const Layer
   const int ntiles = tiles_x * g.H;
   const int n = g.n_planes;
   const int half = (a.scale + (a.scale >> 31)) >> 1;
-  const uint32_t* ref = reinterpret_cast<const uint32_t*>(a.ref);
   const float* Wm = a.warp[0];
   const float w0 = Wm[0], w1 = Wm[1], w2 = Wm[2], w4 = Wm[4], w5 = Wm[5], w6 = Wm[6];
   const int iw = a.ow[0], ih = a.oh[0], x1 = iw - 2, y1 = ih - 2;
   const uint32_t* phase = a.phase[0];
-  const int plane_stride = ih * iw;
   constexpr int kNoRow = INT_MIN;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < ntiles; t += (gridDim.x * blockDim.x) >> 5) {
     const int y = t / tiles_x, xr = ((t - y * tiles_x) << 5) + lane;
@@ -354,22 +392,9 @@ __global__ void __launch_bounds__(256) k_cost_axis(const CostArgs a, const Layer
       for (int d = 0; d < n; d += 8) *reinterpret_cast<uint2*>(out + d) = make_uint2(0u, 0u);
     if (__ballot_sync(0xffffffffu, live) == 0) continue;
     const int xImg = min(a.scale * x + half, a.rw - 1), yImg = min(a.scale * y + half, a.rh - 1);
-    uint32_t ge[3], go[3], re[3][3], ro[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; r++) {  // the reference 3x3 block, rows/columns clamped to the image
-      const int yy = min(max(yImg + r - 1, 0), a.rh - 1);
-      uint32_t yb[3];
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const uint32_t w = __ldg(ref + (size_t)yy * a.rw + min(max(xImg + c - 1, 0), a.rw - 1));
-        yb[c] = w & 0xffu;
-        re[r][c] = w & 0x00ff00ffu;
-        ro[r][c] = (w >> 8) & 0x00ff00ffu;
-      }
-      ge[r] = yb[0] | (yb[2] << 16);
-      go[r] = yb[1];
-    }
-    const GreyRef gr = grey_ref(ge, go);
+    uint32_t rb[3][3];
+    ref_block(a, xImg, yImg, rb);
+    const GreyRef gr = grey_ref(rb);
     const float xf = (float)xImg, yf = (float)yImg;
     int last = 0;
     uint32_t pk0 = 0, pk1 = 0;
@@ -397,8 +422,8 @@ __global__ void __launch_bounds__(256) k_cost_axis(const CostArgs a, const Layer
       const int ix = tx >> 1, iy = ty >> 1;
       if (ix >= 1 && ix < x1 && iy >= 1 && iy < y1) {
         if (live) {
-          const size_t qi = ((size_t)(((ty & 1) << 1) | (tx & 1)) * ih + (iy - 1)) * iw + (ix - 1);
-          last = GREY ? grey_cost(reinterpret_cast<const uint2*>(phase) + qi, iw, gr) : colour_cost(phase + qi, iw, re, ro, a.wq[0]);
+          const size_t qi = (size_t)(ty - 2) * (2 * iw) + (tx - 2);
+          last = GREY ? grey_cost(phase + qi, iw, gr) : colour_cost(phase + qi, iw, rb, a.wq[0]);
         }
       } else if (live) {  // the scalar fallback of the reference would read out of the image
         atomicCAS(err, 0, 7);
@@ -414,7 +439,7 @@ __global__ void __launch_bounds__(256) k_cost_axis(const CostArgs a, const Layer
         const float yz = __fmul_rn(yf, __ldg(g.planes + dj));
         const float fy = __fadd_rn(__fmul_rn(__fadd_rn(zj.y, __fmul_rn(yz, w5)), zj.w), 0.25f);
         const int ty = f2i(__fadd_rn(fy, fy)), iy = ty >> 1;
-        rowoff = (iy >= 1 && iy < y1) ? ((((ty & 1) << 1) * ih) + iy - 1) * iw - 1 : kNoRow;
+        rowoff = (iy >= 1 && iy < y1) ? (ty - 2) * 2 * iw - 2 : kNoRow;
       }
       const int jend = min(32, n - d0);
       for (int j = (d0 == 0 ? 1 : 0); j < jend; j++) {
@@ -426,8 +451,8 @@ __global__ void __launch_bounds__(256) k_cost_axis(const CostArgs a, const Layer
           const float fx = __fadd_rn(__fmul_rn(__fadd_rn(zk.x, __fmul_rn(xz, w0)), zk.w), 0.25f);
           const int tx = f2i(__fadd_rn(fx, fx)), ix = tx >> 1;
           if (ix >= 1 && ix < x1) {
-            const int qi = ro_d + (tx & 1) * plane_stride + ix;
-            last = GREY ? grey_cost(reinterpret_cast<const uint2*>(phase) + qi, iw, gr) : colour_cost(phase + qi, iw, re, ro, a.wq[0]);
+            const int qi = ro_d + tx;
+            last = GREY ? grey_cost(phase + qi, iw, gr) : colour_cost(phase + qi, iw, rb, a.wq[0]);
           }
         }
         put(d, (uint32_t)last);
@@ -1024,21 +1049,9 @@ void launch_phases(const CostArgs& a, cudaStream_t s) {
     if (a.unit)
       k_phase_bytes<<<dim3((unit_pitch(a.ow[k]) / 4 + 127) / 128, a.oh[k]), 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint8_t*>(out));
     else if (a.vcols) k_phase_grey_v<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint2*>(out));
-    else if (grey) k_phase_grey<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], reinterpret_cast<uint2*>(out));
+    else if (grey) k_phase_grey<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], out);
     else k_phase_colour<<<grid, 128, 0, s>>>(a.other[k], a.ow[k], a.oh[k], out);
     count_launches(1);
-  }
-}
-
-template <bool GREY>
-static void launch_rows(int nk, int blocks, const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t* raw, int* err,
-                        cudaStream_t s) {
-  switch (nk) {
-    case 1: k_cost_rows<GREY, 1><<<blocks, 256, 0, s>>>(a, g, zt, raw, err); break;
-    case 2: k_cost_rows<GREY, 2><<<blocks, 256, 0, s>>>(a, g, zt, raw, err); break;
-    case 3: k_cost_rows<GREY, 3><<<blocks, 256, 0, s>>>(a, g, zt, raw, err); break;
-    case 4: k_cost_rows<GREY, 4><<<blocks, 256, 0, s>>>(a, g, zt, raw, err); break;
-    default: k_cost_rows<GREY, kMaxCams - 1><<<blocks, 256, 0, s>>>(a, g, zt, raw, err); break;
   }
 }
 
@@ -1051,7 +1064,9 @@ int launch_cost(const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t
   const int npx = g.W * g.H;
   const bool grey = cost_all_grey(a);
   int kind = 0;
-  if (g.uniform && !cost_small_wide_layer(g.W, g.H, g.n_planes) && g.n_planes % 8 == 0 && a.n_others >= 1 &&
+  bool small_index = true;  // the row kernel's half-pixel positions are below 2^22, its offsets into phase images ints
+  for (int k = 0; k < a.n_others; k++) small_index &= std::max(a.ow[k], a.oh[k]) < 1 << 20 && (size_t)a.ow[k] * a.oh[k] < (size_t)1 << 29;
+  if (g.uniform && (a.axis || small_index) && !cost_small_wide_layer(g.W, g.H, g.n_planes) && g.n_planes % 8 == 0 && a.n_others >= 1 &&
       a.n_others <= kMaxCams - 1) {
     const int tiles = ((g.W + 31) / 32) * g.H;
     int blocks = (tiles + 7) / 8;
@@ -1074,8 +1089,9 @@ int launch_cost(const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t
       else k_cost_axis<false><<<blocks, 256, 0, s>>>(a, g, zt, raw, err);
       kind = 2;
     } else {
-      if (grey) launch_rows<true>(a.n_others, blocks, a, g, zt, raw, err, s);
-      else launch_rows<false>(a.n_others, blocks, a, g, zt, raw, err, s);
+      constexpr int kWarps = kRowsThreads / 32;
+      if (grey) k_cost_rows<true><<<(tiles + kWarps - 1) / kWarps, kRowsThreads, 0, s>>>(a, g, zt, raw, err);
+      else k_cost_rows<false><<<(tiles + kWarps - 1) / kWarps, kRowsThreads, 0, s>>>(a, g, zt, raw, err);
       kind = 1;
     }
   } else {

@@ -37,7 +37,7 @@ struct CostArgs {
   const uint8_t* ref; int rw, rh;  // box-filtered reference image (dense RGBA8)
   int n_others;
   const uint8_t* other[kMaxCams];
-  const uint32_t* phase[kMaxCams];  // per other camera: four half-pixel phase images, [4][oh][ow] of uint2 (grey) or u32
+  const uint32_t* phase[kMaxCams];  // per other camera: four half-pixel phase images, [4][oh][ow] of u32 (vcols: uint2)
   int ow[kMaxCams], oh[kMaxCams];
   float warp[kMaxCams][16];
   uint16_t wq[kMaxCams][4];

@@ -400,7 +400,7 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     ca.norm_mul = cost_unit_norm(ca.norm);
     ca.unit = Wm[0] == Wm[10] && Wm[5] == Wm[10] && Wm[14] == 0.0f && Wm[10] != 0.0f && ca.norm_mul ? 1 : 0;
   }
-  const size_t phase_words = cost_all_grey(ca) ? 8 : 4;  // per pixel: four phases of {u16 pairs} (grey) or RGBA words
+  const size_t phase_words = ca.vcols ? 8 : 4;  // per pixel: four phases of a word, or of the vertical triples' u16 pairs
   for (int k = 0; k < ca.n_others; k++) {  // the half-pixel phase images of the other cameras
     uint32_t* ph = nullptr;
     const size_t words = ca.unit ? cost_unit_phase_bytes(ca.ow[k], ca.oh[k], L->n) / 4 : phase_words * ca.ow[k] * ca.oh[k];
