@@ -297,9 +297,9 @@ struct CensusLines {
   CensusPairs ps;
 };
 
-// unpack8 with the disparities past D raised by kBeyond
+// unpack with the disparities past D raised by kBeyond
 LUX_DEV void unpack_cost(L4& v, uint2 b, const L4& pad) {
-  unpack8(v, b);
+  unpack(v, b);
 #pragma unroll
   for (int k = 0; k < 4; k++) v.r[k] |= pad.r[k];
 }
@@ -324,7 +324,7 @@ LUX_DEV void census_forward(const CensusLines& a, const CensusPair& pr, int wi, 
   const int NS = line_len(a, P, line);
   Walk w = walk_at(a, P, line_first(a, P, line), 1), ws = w;
   const L4 pad = pad_of(gl, pr.D, kBeyond);
-  RawRing rr(ring + lane, in);
+  RawRing<8> rr(ring + lane, in);
   L4 L;
   uint32_t md;
   set_zero(L, md);

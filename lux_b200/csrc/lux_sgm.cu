@@ -441,7 +441,7 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     if (!forced) {
       const TunedForm t = tuned_form(W, H, L->n, p.tile);
       // The lines form is faster than the other three at every size (4160x3120 D=256: 15.4 against 17.6 ms; 1040x780
-      // D=64: 0.66 against 4.5 ms; 520x390 D=32: 0.29 against 2.4 ms) but never holds pass +1's aggregates alone and waits on nothing (debug_stall).
+      // D=64: 0.64 against 4.5 ms; 520x390 D=32: 0.26 against 2.4 ms) but never holds pass +1's aggregates alone and waits on nothing (debug_stall).
       if (!(flags & LUX_LAYER_KEEP_PASS1) && !t.set_by_caller && ctx->stall_block < 0 && lines_supported(W, L->n)) {
         form = 4;
       } else {

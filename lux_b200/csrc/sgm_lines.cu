@@ -7,12 +7,12 @@
 // that the lines of a path are equally long (to one step) and their addresses linear. On the fast path no sum saturates,
 // so the aggregate is the sum of the eight paths in any order.
 //
-// A lane holds eight planes p0..p7 of its line as u16 pairs (p0, p4), (p1, p5), (p2, p6), (p3, p7): the planes before and
+// A lane holds K = 8 planes p0..p7 of its line as u16 pairs (p0, p4), (p1, p5), (p2, p6), (p3, p7) (or K = 4, below): the planes before and
 // after a pair's are the neighbouring registers', and only the two at the ends take a byte permute. The aggregates keep
-// this order within every octet of planes until the last read, which puts them in order where they are kept. A step is 47
+// this order within every K planes until the last read, which puts them in order where they are kept. A step is 47
 // cycles of a scheduler (44.3 without its loads; 53.7 with pairs of adjacent planes, 62 with the DPX min/add forms): the
 // 16-bit minima and permutes bound it, so the adds are multiply-adds by a kernel-argument one, which issue elsewhere. A
-// line takes GL = 4, 8, 16 or 32 lanes (planes / 8, rounded
+// line takes GL = 4, 8, 16 or 32 lanes (planes / K, rounded
 // up to a power of two), so a warp carries 32 / GL neighbouring lines. Two forms, chosen by size (run_sgm_lines):
 //   * small layers: the four paths of a pass in one launch, each adding its L into the aggregates by reductions in L2 (four
 //     u16 sums in a 64-bit add, none of which can carry). A pass is as long as one line: latency is what such a layer costs.
@@ -66,30 +66,60 @@ struct LineArgs {
   int keep_agg;
 };
 
-LUX_DEV void set_init(L4& v, uint32_t& md) {
-  v.r[0] = v.r[1] = v.r[2] = v.r[3] = kInit2;
+template <int K>
+LUX_DEV void set_init(Planes<K>& v, uint32_t& md) {
+#pragma unroll
+  for (int i = 0; i < K / 2; i++) v.r[i] = kInit2;
   md = kInit2;
 }
-LUX_DEV uint4 in_order(const L4& v) {  // planes 0..7 one after the other, as the aggregates are kept
-  return make_uint4(__byte_perm(v.r[0], v.r[1], 0x5410), __byte_perm(v.r[2], v.r[3], 0x5410), __byte_perm(v.r[0], v.r[1], 0x7632),
-                    __byte_perm(v.r[2], v.r[3], 0x7632));
+// Planes 0..K-1 one after the other, as the aggregates are kept.
+template <int K>
+LUX_DEV Planes<K> in_order(const Planes<K>& v) {
+  Planes<K> o;
+#pragma unroll
+  for (int i = 0; i < K / 2; i++) {
+    constexpr int N = K / 2;
+    const int j = 2 * i % N;  // (pairs of planes 2i, 2i + 1: in the low halves of two registers, then in the high ones)
+    o.r[i] = __byte_perm(v.r[j], v.r[j + 1 < N ? j + 1 : j], i < N / 2 ? 0x5410 : 0x7632);
+  }
+  return o;
+}
+// A lane's planes in global memory, 2K bytes.
+template <int K>
+LUX_DEV Planes<K> load_planes(const uint16_t* p) {
+  Planes<K> v;
+  if constexpr (K == 8) v = as_l4(__ldcg(reinterpret_cast<const uint4*>(p)));
+  else {
+    const uint2 t = __ldcg(reinterpret_cast<const uint2*>(p));
+    v.r[0] = t.x;
+    v.r[1] = t.y;
+  }
+  return v;
+}
+template <int K>
+LUX_DEV void store_planes(uint16_t* p, const Planes<K>& v) {
+  if constexpr (K == 8) __stcg(reinterpret_cast<uint4*>(p), as_uint4(v));
+  else __stcg(reinterpret_cast<uint2*>(p), make_uint2(v.r[0], v.r[1]));
 }
 
-// Adds eight u16 sums in L2. No u16 of the aggregates can carry into the next one (every path's L is below 2000).
-LUX_DEV void red_add8(uint16_t* p, const L4& v) {
-  const unsigned long long a = v.r[0] | ((unsigned long long)v.r[1] << 32), b = v.r[2] | ((unsigned long long)v.r[3] << 32);
-  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(a));  // nothing in the kernel reads the sums
-  asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p + 4), "l"(b));
+// Adds a lane's u16 sums in L2. No u16 of the aggregates can carry into the next one (every path's L is below 2000).
+template <int K>
+LUX_DEV void red_add(uint16_t* p, const Planes<K>& v) {  // nothing in the kernel reads the sums
+#pragma unroll
+  for (int i = 0; i < K / 2; i += 2)
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p + 2 * i), "l"(v.r[i] | ((unsigned long long)v.r[i + 1] << 32)));
 }
 
-// A kept state (kState u16 apart): lane gl of the line holds planes 8gl..8gl+7.
-LUX_DEV void put_state(uint16_t* base, uint16_t* mins, size_t i, const L4& L, uint32_t md, int gl, bool in) {
-  if (in) __stcg(reinterpret_cast<uint4*>(base + i * kState) + gl, as_uint4(L));
+// A kept state (kState u16 apart): lane gl of the line holds planes K·gl to K·gl + K - 1.
+template <int K>
+LUX_DEV void put_state(uint16_t* base, uint16_t* mins, size_t i, const Planes<K>& L, uint32_t md, int gl, bool in) {
+  if (in) store_planes<K>(base + i * kState + gl * K, L);
   if (gl == 0) __stcg(mins + i, (unsigned short)(md & 0xffffu));
 }
-LUX_DEV void get_state(const uint16_t* base, const uint16_t* mins, size_t i, L4& L, uint32_t& md, int gl, bool in) {
+template <int K>
+LUX_DEV void get_state(const uint16_t* base, const uint16_t* mins, size_t i, Planes<K>& L, uint32_t& md, int gl, bool in) {
   set_init(L, md);
-  if (in) L = as_l4(__ldcg(reinterpret_cast<const uint4*>(base + i * kState) + gl));
+  if (in) L = load_planes<K>(base + i * kState + gl * K);
   md = dup16(__ldcg(mins + i));
 }
 
@@ -104,7 +134,8 @@ LUX_DEV uint32_t p2_between(const LineArgs& a, float4 g, float4 m) {
 LUX_DEV uint32_t p2_entry(const LineArgs& a, int pix, int p) { return __ldg(reinterpret_cast<const uint16_t*>(a.p2t + pix) + p); }
 
 // What pass -1 reads above its first row for path p (1..3) at column x: pass +1's state of row y_b at x + dx.
-LUX_DEV void edge_start(const LineArgs& a, int p, int x, L4& L, uint32_t& md, uint32_t& P2, int gl, bool in) {
+template <int K>
+LUX_DEV void edge_start(const LineArgs& a, int p, int x, Planes<K>& L, uint32_t& md, uint32_t& P2, int gl, bool in) {
   const int xe = x + (p == 1 ? 1 : p == 3 ? -1 : 0);
   set_init(L, md);
   P2 = 0;
@@ -116,24 +147,24 @@ LUX_DEV void edge_start(const LineArgs& a, int p, int x, L4& L, uint32_t& md, ui
 // A column's path-2 chain of one pass by a whole warp, its L added by reductions to sums (image row r at r·stride·n:
 // the column's aggregates, or a buffer of its own). SPECIAL: the pass's
 // last column (x = W-1 of pass +1, x = 0 of pass -1) with the reference's revisits (revisit_schedule.h). In every T-row
-// band of nr rows it visits rows 0..v-1 (v = min(K, nr), K = T - (W-1) mod T), then revisits rows 0..v-1, then visits the
+// band of nr rows it visits rows 0..v-1 (v = min(R, nr), R = T - (W-1) mod T), then revisits rows 0..v-1, then visits the
 // rest, each reading what the step before left: one chain, except that a band's first revisit reads the newest state of
 // the line-buffer half it looks into, which is the last visit's for even v and the one before it for odd v (for v = 1 in
 // the first band: the pass's boundary). A revisit also adds its path 3, which restarts from the margin and so equals the
 // raw cost.
-template <bool BWD, bool SPECIAL>
-LUX_DEV void column_chain(const LineArgs& a, int x, int lane, uint2* ring, uint16_t* sums, int stride) {
+template <int K, bool BWD, bool SPECIAL>
+LUX_DEV void column_chain(const LineArgs& a, int x, int lane, typename RawOf<K>::type* ring, uint16_t* sums, int stride) {
   const int W = a.W, H = a.H, n = a.n, T = a.T;
-  const bool in = lane * 8 < n, first = lane == 0, last = lane * 8 + 8 == n;
-  const int K = SPECIAL ? T - (W - 1) % T : 0;
-  const int full = T + K;  // steps of a whole band
+  const bool in = lane * K < n, first = lane == 0, last = lane * K + K == n;
+  const int R = SPECIAL ? T - (W - 1) % T : 0;
+  const int full = T + R;  // steps of a whole band
   const int tail = H % T;  // rows of a partial last band
-  const int steps = SPECIAL ? (H / T) * full + (tail ? tail + min(K, tail) : 0) : H;
+  const int steps = SPECIAL ? (H / T) * full + (tail ? tail + min(R, tail) : 0) : H;
   // step s of the chain: its row of the pass; rev: a revisit; start: a band's first revisit
   auto row_of = [&](int s, bool& rev, bool& start) {
     rev = start = false;
     if (!SPECIAL) return s;
-    const int j = s / full, o = s - j * full, base = j * T, v = min(K, min(T, H - base));
+    const int j = s / full, o = s - j * full, base = j * T, v = min(R, min(T, H - base));
     rev = o >= v && o < 2 * v;
     start = o == v;
     return o < v ? base + o : base + o - v;
@@ -151,16 +182,21 @@ LUX_DEV void column_chain(const LineArgs& a, int x, int lane, uint2* ring, uint1
     const int t = rv & 0x1fffffff;
     return t > 0 ? p2_entry(a, BWD ? pix(t - 1) : pix(t), 2) : 0u;
   };
-  RawRing rr(ring + lane, in);
+  // A batch's costs by eight bytes a lane, rows one after the other (a lone warp waits for its instructions more than for
+  // anything else: 92 batches of 738 steps at 877 instructions took 146 us).
+  using Raw = typename RawOf<K>::type;
+  RawRing<K> rr(ring + lane, in);
+  const int oct = n >> 3, per_oct = (65536 + oct - 1) / oct;
   auto stage = [&](int b, int rv) {
-#pragma unroll
-    for (int i = 0; i < kBatch; i++) {
-      const int t = __shfl_sync(0xffffffffu, rv, i) & 0x1fffffff;
-      if (in) rr.stage(b, i, a.raw + (size_t)pix(t) * n + lane * 8);
+    for (int c0 = 0; c0 < kBatch * oct; c0 += 32) {
+      const int c = c0 + lane, i = (c * per_oct) >> 16, part = c - i * oct;
+      const int t = __shfl_sync(0xffffffffu, rv, i & (kBatch - 1)) & 0x1fffffff;
+      if (i < kBatch)
+        cp_async8(reinterpret_cast<char*>(ring + ((b & 1) * kBatch + i) * 32) + part * 8, a.raw + (size_t)pix(t) * n + part * 8);
     }
     cp_async_commit();
   };
-  L4 L, Lp;  // the state, and the state one step before
+  Planes<K> L, Lp;  // the state, and the state one step before
   uint32_t md, mp, P2start = 0;
   set_init(L, md);
   if (BWD) edge_start(a, 2, x, L, md, P2start, lane, in);
@@ -173,28 +209,35 @@ LUX_DEV void column_chain(const LineArgs& a, int x, int lane, uint2* ring, uint1
   const int nb = (steps + kBatch - 1) / kBatch;
   for (int b = 0; b < nb; b++) {
     cp_async_wait<1>();
+    __syncwarp();  // (a lane's costs were copied by others)
     const int len = min(kBatch, steps - b * kBatch);
-    uint2 rb[kBatch];
+    Raw rb[kBatch];
 #pragma unroll
     for (int i = 0; i < kBatch; i++) rb[i] = rr.get(b, i);
     const uint32_t pd = dup16(pv);
     // a whole batch with no band's first revisit, no state to keep and not the pass's start
     const bool plain = b > 0 && len == kBatch &&
                        !__any_sync(0xffffffffu, (rv & (1 << 30)) || (!BWD && (rv & 0x1fffffff) == a.y_b));
-    if (plain) {
+    if (plain) {  // its rows follow one another
+      uint32_t p2[kBatch];
 #pragma unroll
-      for (int i = 0; i < kBatch; i++) {
-        const int ev = __shfl_sync(0xffffffffu, rv, i), t = ev & 0x1fffffff;
-        L4 raw2;
-        unpack8(raw2, rb[i]);
+      for (int i = 0; i < kBatch; i++) p2[i] = __shfl_sync(0xffffffffu, pd, i);
+      const uint32_t revs = SPECIAL ? __ballot_sync(0xffffffffu, rv & (1 << 29)) : 0u;
+      const int t0 = __shfl_sync(0xffffffffu, rv, 0) & 0x1fffffff;
+      uint16_t* ap = sums + (size_t)(BWD ? H - 1 - t0 : t0) * stride * n + lane * K;
+      const long long ds = (long long)(BWD ? -stride : stride) * n;
+#pragma unroll
+      for (int i = 0; i < kBatch; i++, ap += ds) {
+        Planes<K> raw2;
+        unpack(raw2, rb[i]);
         Lp = L;
         mp = md;
-        line_step<32>(L, md, raw2, __shfl_sync(0xffffffffu, pd, i), a, first, last);
-        const uint32_t twice = SPECIAL ? (uint32_t)ev >> 29 : 0u;  // bit 29 alone here
-        L4 s;
+        line_step<32>(L, md, raw2, p2[i], a, first, last);
+        const uint32_t twice = (revs >> i) & 1u;
+        Planes<K> s;
 #pragma unroll
-        for (int k = 0; k < 4; k++) s.r[k] = raw2.r[k] * twice + L.r[k];
-        if (in) red_add8(sums + (size_t)(BWD ? H - 1 - t : t) * stride * n + lane * 8, s);
+        for (int k = 0; k < K / 2; k++) s.r[k] = raw2.r[k] * twice + L.r[k];
+        if (in) red_add(ap, s);
       }
     } else {
 #pragma unroll 1
@@ -203,7 +246,7 @@ LUX_DEV void column_chain(const LineArgs& a, int x, int lane, uint2* ring, uint1
         uint32_t p2 = __shfl_sync(0xffffffffu, pv, i);
         if (b == 0 && i == 0) p2 = P2start;
         if (SPECIAL && (ev & (1 << 30))) {
-          const int v = min(K, min(T, H - t)), src = (v & 1) ? t + v - 2 : t + v - 1;
+          const int v = min(R, min(T, H - t)), src = (v & 1) ? t + v - 2 : t + v - 1;
           const float4 g = guide_at(a, x, BWD ? H - 1 - t : t);
           if (v & 1) {
             L = Lp;
@@ -217,18 +260,18 @@ LUX_DEV void column_chain(const LineArgs& a, int x, int lane, uint2* ring, uint1
             if (BWD) edge_start(a, 2, x, L, md, p2, lane, in);
           }
         }
-        L4 raw2;
-        unpack8(raw2, rr.get(b, i));
+        Planes<K> raw2;
+        unpack(raw2, rr.get(b, i));
         Lp = L;
         mp = md;
         line_step<32>(L, md, raw2, dup16(p2), a, first, last);
         if (in) {
-          L4 s = L;
+          Planes<K> s = L;
           if (SPECIAL && (ev & (1 << 29))) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) s.r[k] += raw2.r[k];
+            for (int k = 0; k < K / 2; k++) s.r[k] += raw2.r[k];
           }
-          red_add8(sums + (size_t)(BWD ? H - 1 - t : t) * stride * n + lane * 8, s);
+          red_add(sums + (size_t)(BWD ? H - 1 - t : t) * stride * n + lane * K, s);
         }
         if (!BWD && t == a.y_b) put_state(a.edge, a.edge_min, (size_t)1 * W + x, L, md, lane, in);  // the last writer counts
       }
@@ -246,24 +289,25 @@ LUX_DEV void column_chain(const LineArgs& a, int x, int lane, uint2* ring, uint1
 
 // Paths 0 and 1 of pass PASS's revisits R(c, y), a warp each: their sources are states of column c-1, pass +1's final row,
 // or never-written slots.
-template <bool BWD>
+template <int K, bool BWD>
 __global__ void __launch_bounds__(128) k_lines_revisit(const LineArgs a) {
   const int lane = threadIdx.x & 31, k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (k >= a.n_rev[BWD ? 1 : 0]) return;
   const int W = a.W, H = a.H, n = a.n;
-  const bool in = lane * 8 < n, first = lane == 0, last = lane * 8 + 8 == n;
+  const bool in = lane * K < n, first = lane == 0, last = lane * K + K == n;
   const int* sch = a.sched[BWD ? 1 : 0];
   const int y = sch[3 * H + k];
   const int xc = BWD ? 0 : W - 1, xn = BWD ? 1 : W - 2;  // columns c and c-1 of the pass
   auto row = [&](int t) { return BWD ? H - 1 - t : t; };
   const float4 g = guide_at(a, xc, row(y));
   const size_t pi = (size_t)row(y) * W + xc;
-  L4 raw2, sum{};
-  unpack8(raw2, in ? __ldg(reinterpret_cast<const uint2*>(a.raw + pi * n) + lane) : kPastRaw);
+  Planes<K> raw2, sum{};
+  using Raw = typename RawOf<K>::type;
+  unpack(raw2, in ? __ldg(reinterpret_cast<const Raw*>(a.raw + pi * n) + lane) : RawOf<K>::past());
 #pragma unroll
   for (int p = 0; p < 2; p++) {
     const int e = sch[p * H + y], kind = src_kind(e);
-    L4 L;
+    Planes<K> L;
     uint32_t md, p2 = 0;
     set_init(L, md);
     if (kind == kSrcEdge) {
@@ -277,26 +321,27 @@ __global__ void __launch_bounds__(128) k_lines_revisit(const LineArgs a) {
     }
     line_step<32>(L, md, raw2, dup16(p2), a, first, last);
 #pragma unroll
-    for (int i = 0; i < 4; i++) sum.r[i] += L.r[i];
+    for (int i = 0; i < K / 2; i++) sum.r[i] += L.r[i];
     // R(y_b) is what pass -1 will read at the last column
     if (!BWD && p == 1 && (sch[2 * H + y] & 1)) put_state(a.edge, a.edge_min, xc, L, md, lane, in);
   }
-  if (in) red_add8(a.agg + pi * n + lane * 8, sum);
+  if (in) red_add(a.agg + pi * n + lane * K, sum);
 }
 
 // Small layers: the four paths of a pass, one launch. Warp 0 takes the special column's path 2, the others 32 / GL lines.
 // Latency-bound: a layer this small has one to sixteen warps an SM, and a pass lasts as long as its longest chain.
-template <int GL, bool BWD>
+template <int GL, int K, bool BWD>
 __global__ void __launch_bounds__(64) k_lines_pass(const LineArgs a) {
   constexpr int LPW = 32 / GL;
-  __shared__ uint2 s_ring[2][2 * kBatch * 32];
+  using Raw = typename RawOf<K>::type;
+  __shared__ Raw s_ring[2][2 * kBatch * 32];
   const int W = a.W, H = a.H, n = a.n;
   const int lane = threadIdx.x & 31, gl = lane & (GL - 1), grp = lane / GL;
-  uint2* ring = s_ring[threadIdx.x >> 5];
+  Raw* ring = s_ring[threadIdx.x >> 5];
   int wi = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) - 1;
   const int xc = BWD ? 0 : W - 1;  // the pass's last column
   if (wi < 0) {
-    column_chain<BWD, true>(a, xc, lane, ring, a.agg + (size_t)xc * n, W);
+    column_chain<K, BWD, true>(a, xc, lane, ring, a.agg + (size_t)xc * n, W);
     return;
   }
   int p = 1;
@@ -310,11 +355,11 @@ __global__ void __launch_bounds__(64) k_lines_pass(const LineArgs a) {
   if (wi * LPW >= NL) return;
   const int line0 = wi * LPW + grp, line = min(line0, NL - 1);
   const bool valid = line0 < NL && !(p == 2 && line0 == xc);
-  const bool inl = gl * 8 < n, in = valid && inl, first = gl == 0, last = gl * 8 + 8 == n;
+  const bool inl = gl * K < n, in = valid && inl, first = gl == 0, last = gl * K + K == n;
   const int NS = line_len(a, p, line);
   Walk w = walk_at(a, p, line_first(a, p, line) + (BWD ? (NS - 1) * line_step_of(p, W) : 0), BWD ? -1 : 1), ws = w;
-  RawRing rr(ring + lane, in);
-  L4 L;
+  RawRing<K> rr(ring + lane, in);
+  Planes<K> L;
   uint32_t md, p2prev = 0;
   set_init(L, md);
   if (BWD && p > 0 && w.pi >= W * (H - 1)) edge_start(a, p, w.pi - W * (H - 1), L, md, p2prev, gl, inl);
@@ -349,19 +394,21 @@ __global__ void __launch_bounds__(64) k_lines_pass(const LineArgs a) {
     if (p == 0) odd |= t0 + kBatch > W - 2;
     if (!BWD && p > 0) odd |= a.y_b >= 0 && w.pi + w.step * (kBatch - 1) >= a.y_b * W;
     if (!__any_sync(0xffffffffu, odd)) {
-      uint2 rb[kBatch];
+      Raw rb[kBatch];
 #pragma unroll
       for (int i = 0; i < kBatch; i++) rb[i] = rr.get(b, i);
-      uint16_t* ap = a.agg + (size_t)w.pi * n + gl * 8;
+      uint32_t p2[kBatch];  // (a shuffle between the steps would be waited for)
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) p2[i] = p2_at(i);
+      uint16_t* ap = a.agg + (size_t)w.pi * n + gl * K;
       const long long ds = (long long)w.step * n;
 #pragma unroll
       for (int i = 0; i < kBatch; i++, ap += ds) {
-        L4 raw2;
-        unpack8(raw2, rb[i]);
-        const uint32_t p2 = p2_at(i);
-        line_step<GL>(L, md, raw2, BWD ? p2prev : p2, a, first, last);
-        p2prev = p2;
-        if (in) red_add8(ap, L);
+        Planes<K> raw2;
+        unpack(raw2, rb[i]);
+        line_step<GL>(L, md, raw2, BWD ? p2prev : p2[i], a, first, last);
+        p2prev = p2[i];
+        if (in) red_add(ap, L);
       }
     } else {
       int x = w.x, pi = w.pi;
@@ -370,12 +417,12 @@ __global__ void __launch_bounds__(64) k_lines_pass(const LineArgs a) {
         const bool live = t0 + i < NS;
         // a new line: the pixel at the side the diagonal enters by (but pass -1's last row starts from the edge state)
         if (w.dx != 0 && t0 + i > 0 && x == (w.dx > 0 ? 0 : W - 1)) set_init(L, md);
-        L4 raw2;
-        unpack8(raw2, rr.get(b, i));
+        Planes<K> raw2;
+        unpack(raw2, rr.get(b, i));
         const uint32_t p2 = p2_at(i);
         line_step<GL>(L, md, raw2, BWD ? p2prev : p2, a, first, last);
         p2prev = p2;
-        if (in && live) red_add8(a.agg + (size_t)pi * n + gl * 8, L);
+        if (in && live) red_add(a.agg + (size_t)pi * n + gl * K, L);
         const int y = p == 0 ? line : p == 2 ? (BWD ? H - 1 - t0 - i : t0 + i) : pi / W;
         if (p < 2) {  // N(c-1): paths 0 and 1 are revisit sources
           const bool at = pi - y * W == (BWD ? 1 : W - 2);
@@ -397,19 +444,19 @@ __global__ void __launch_bounds__(64) k_lines_pass(const LineArgs a) {
   cp_async_wait<0>();
 }
 
-template <int GL>
+template <int GL, int K>
 __global__ void __launch_bounds__(256) k_lines_wta(const LineArgs a) {
   constexpr int LPW = 32 / GL;
   const int lane = threadIdx.x & 31, gl = lane & (GL - 1), grp = lane / GL;
   const int npx = a.W * a.H, nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int p0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * LPW; p0 < npx; p0 += nwarps * LPW) {
     const int pi = p0 + grp;
-    const bool in = pi < npx && gl * 8 < a.n;
-    L4 s{};
-    if (in) s = as_l4(__ldcs(reinterpret_cast<const uint4*>(a.agg + (size_t)pi * a.n) + gl));
+    const bool in = pi < npx && gl * K < a.n;
+    Planes<K> s{};
+    if (in) s = load_planes<K>(a.agg + (size_t)pi * a.n + gl * K);
     const int arg = wta_line<GL>(s, gl, lane, in);
     if (in && gl == 0) a.depth[pi] = __ldg(a.planes + arg);
-    if (a.keep_agg && in) __stcs(reinterpret_cast<uint4*>(a.agg + (size_t)pi * a.n) + gl, in_order(s));
+    if (a.keep_agg && in) store_planes<K>(a.agg + (size_t)pi * a.n + gl * K, in_order(s));
   }
 }
 
@@ -428,7 +475,7 @@ LUX_DEV void ckpt_lines(const LineArgs& a, int wi, uint2* ring, uint16_t* ckpt, 
   const bool in = valid && gl * 8 < n, first = gl == 0, last = gl * 8 + 8 == n;
   const int NS = line_len(a, P, line);
   Walk w = walk_at(a, P, line_first(a, P, line), 1), ws = w;
-  RawRing rr(ring + lane, in);
+  RawRing<8> rr(ring + lane, in);
   L4 L;
   uint32_t md;
   set_init(L, md);
@@ -458,7 +505,7 @@ LUX_DEV void ckpt_lines(const LineArgs& a, int wi, uint2* ring, uint16_t* ckpt, 
 #pragma unroll
       for (int i = 0; i < kBatch; i++) {
         L4 raw2;
-        unpack8(raw2, rb[i]);
+        unpack(raw2, rb[i]);
         line_step<GL>(L, md, raw2, __shfl_sync(0xffffffffu, pv, i, GL), a, first, last);
       }
     } else {
@@ -468,7 +515,7 @@ LUX_DEV void ckpt_lines(const LineArgs& a, int wi, uint2* ring, uint16_t* ckpt, 
         const bool live = valid && t0 + i < NS;
         if ((P == 1 && x == 0) || (P == 3 && x == W - 1)) set_init(L, md);
         L4 raw2;
-        unpack8(raw2, rr.get(b, i));
+        unpack(raw2, rr.get(b, i));
         line_step<GL>(L, md, raw2, __shfl_sync(0xffffffffu, pv, i, GL), a, first, last);
         const int y = P == 0 ? line : P == 2 ? t0 + i : pi / W;
         if (P < 2 && live && pi - y * W == W - 2) put_state(a.cs[0], a.cs_min[0], (size_t)y * 2 + P, L, md, gl, in);
@@ -574,7 +621,7 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
 #pragma unroll
       for (int i = 0; i < kSeg; i++) {
         L4 raw2;
-        unpack8(raw2, rawp[i * 32]);
+        unpack(raw2, rawp[i * 32]);
         line_step<GL>(F, fd, raw2, __shfl_sync(0xffffffffu, p2v, i, GL), a, first, last);
         add_fwd(i);
       }
@@ -584,7 +631,7 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
       for (int i = 0; i < kSeg; i++) {
         if ((P == 1 && x == 0) || (P == 3 && x == W - 1)) set_init(F, fd);
         L4 raw2;
-        unpack8(raw2, rawp[i * 32]);
+        unpack(raw2, rawp[i * 32]);
         line_step<GL>(F, fd, raw2, __shfl_sync(0xffffffffu, p2v, i, GL), a, first, last);
         add_fwd(i);
         x += dx;
@@ -604,7 +651,7 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
       if (MODE != 2) {
         if (in && live) __stcs(reinterpret_cast<uint4*>(ap), as_uint4(s));
       } else {
-        if (a.keep_agg && in && live) __stcs(reinterpret_cast<uint4*>(ap), in_order(s));
+        if (a.keep_agg && in && live) __stcs(reinterpret_cast<uint4*>(ap), as_uint4(in_order(s)));
         const int arg = wta_line<GL>(s, gl, lane, gl * 8 < n);
         if ((gl & (kSeg - 1)) == i) win = arg;
       }
@@ -616,7 +663,7 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
 #pragma unroll
       for (int i = kSeg - 1; i >= 0; i--, ap -= ds, rq -= ds) {
         L4 raw2;
-        unpack8(raw2, rawp[i * 32]);
+        unpack(raw2, rawp[i * 32]);
         line_step<GL>(B, bd, raw2, p2back, a, first, last);
         p2back = __shfl_sync(0xffffffffu, p2v, i, GL);
         put(i, ap, true);
@@ -639,7 +686,7 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
           set_init(B, bd);  // a new line: pass -1 comes in at the side the diagonal left by
         }
         L4 raw2;
-        unpack8(raw2, rawp[i * 32]);
+        unpack(raw2, rawp[i * 32]);
         line_step<GL>(B, bd, raw2, p2back, a, first, last);
         p2back = __shfl_sync(0xffffffffu, p2v, i, GL);
         put(i, a.agg + (size_t)pi * n + gl * 8, live);
@@ -683,12 +730,12 @@ __global__ void __launch_bounds__(64, 16) k_lines_walk(const LineArgs a) {
       const int x = wib == 0 ? a.W - 1 : 0;
       if (NEXT == 2) {
         uint16_t* sums = a.col_sums + (size_t)wib * a.H * a.n;
-        if (wib == 0) column_chain<false, true>(a, x, lane, ring, sums, 1);
-        else column_chain<false, false>(a, x, lane, ring, sums, 1);
+        if (wib == 0) column_chain<8, false, true>(a, x, lane, ring, sums, 1);
+        else column_chain<8, false, false>(a, x, lane, ring, sums, 1);
       } else {
         uint16_t* sums = a.agg + (size_t)x * a.n;
-        if (wib == 0) column_chain<true, false>(a, x, lane, ring, sums, a.W);
-        else column_chain<true, true>(a, x, lane, ring, sums, a.W);
+        if (wib == 0) column_chain<8, true, false>(a, x, lane, ring, sums, a.W);
+        else column_chain<8, true, true>(a, x, lane, ring, sums, a.W);
       }
       return;
     }
@@ -709,17 +756,19 @@ __global__ void k_lines_columns(const LineArgs a) {
   if (i >= 2 * a.H * oct) return;
   const int c = i / (a.H * oct), j = i - c * a.H * oct, y = j / oct;
   const L4 v = as_l4(__ldcg(reinterpret_cast<const uint4*>(a.col_sums) + i));
-  red_add8(a.agg + ((size_t)y * a.W + (c == 0 ? a.W - 1 : 0)) * a.n + (j - y * oct) * 8, v);
+  red_add(a.agg + ((size_t)y * a.W + (c == 0 ? a.W - 1 : 0)) * a.n + (j - y * oct) * 8, v);
 }
 
 struct LinesLayout {
   size_t ckpt[2], ckpt_min[2], col_sums, edge, edge_min, cs, cs_min, sched, p2t, total;
 };
-// The small form's eight reductions a value cost 9 us a million planes and pixels at any size; the large form moves less
-// but walks path after path. Small against large, ms: 1431x1073 D=120 1.6 / 2.2, 2080x1560 D=64 1.8 / 2.7, 1431x1073 D=200
-// 3.0 / 2.3, 2080x1560 D=128 3.7 / 3.4. With 32 planes or fewer the large form's lines leave lanes idle: 4160x3120 D=32
-// 4.2 / 5.6.
-bool small_form(int W, int H, int n) { return W < 2 * kSeg || n <= 32 || (size_t)W * H * n < (size_t)240 << 20; }
+// The small form's eight reductions a value cost 8 us a million planes and pixels at any size; the large form moves less
+// but walks path after path. Small against large, ms: 2080x1560 D=64 1.6 / 2.7, D=96 2.5 / 2.9, D=128 3.0 / 3.1, 3000x2000 D=64
+// 3.3 / 3.5, 4160x3120 D=40 5.1 / 5.5, D=64 6.6 / 5.8, D=128 12.8 / 9.0; past 128 planes, where a lane holds eight in either
+// form, 1431x1073 D=200 3.0 / 2.3. With 32 planes or fewer the large form's lines leave lanes idle: 4160x3120 D=32 3.1 / 5.6.
+bool small_form(int W, int H, int n) {
+  return W < 2 * kSeg || n <= 32 || (size_t)W * H * n < (size_t)(n <= 128 ? 480 : 240) << 20;
+}
 
 LinesLayout lines_layout(int W, int H, int n) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -742,18 +791,18 @@ LinesLayout lines_layout(int W, int H, int n) {
   return s;
 }
 
-template <int GL>
+template <int GL, int K>
 void run_small(const LineArgs& a, cudaStream_t s) {
   constexpr int LPW = 32 / GL;
   auto warps_of = [](int lines) { return (lines + LPW - 1) / LPW; };
   const int blocks = (1 + warps_of(a.W + 1) + warps_of(a.W) + warps_of(a.W - 1) + warps_of(a.H) + 1) / 2;
   cudaMemsetAsync(a.agg, 0, (size_t)a.W * a.H * a.n * 2, s);
-  k_lines_pass<GL, false><<<blocks, 64, 0, s>>>(a);
-  if (a.n_rev[0]) k_lines_revisit<false><<<(a.n_rev[0] + 3) / 4, 128, 0, s>>>(a);
-  k_lines_pass<GL, true><<<blocks, 64, 0, s>>>(a);
-  if (a.n_rev[1]) k_lines_revisit<true><<<(a.n_rev[1] + 3) / 4, 128, 0, s>>>(a);
+  k_lines_pass<GL, K, false><<<blocks, 64, 0, s>>>(a);
+  if (a.n_rev[0]) k_lines_revisit<K, false><<<(a.n_rev[0] + 3) / 4, 128, 0, s>>>(a);
+  k_lines_pass<GL, K, true><<<blocks, 64, 0, s>>>(a);
+  if (a.n_rev[1]) k_lines_revisit<K, true><<<(a.n_rev[1] + 3) / 4, 128, 0, s>>>(a);
   const int wta = (a.W * a.H + 8 * LPW - 1) / (8 * LPW);
-  k_lines_wta<GL><<<std::min(wta, 148 * 8), 256, 0, s>>>(a);
+  k_lines_wta<GL, K><<<std::min(wta, 148 * 8), 256, 0, s>>>(a);
   count_launches(3 + (a.n_rev[0] > 0) + (a.n_rev[1] > 0));
 }
 
@@ -773,9 +822,9 @@ void run_large(const LineArgs& a, cudaStream_t s) {
   run_walk<GL, -1, 0, 0>(a, s);
   run_walk<GL, 0, 0, 1>(a, s);
   // pass -1's diagonals from the last column start at what the last revisit left there
-  if (a.n_rev[0]) k_lines_revisit<false><<<(a.n_rev[0] + 3) / 4, 128, 0, s>>>(a);
+  if (a.n_rev[0]) k_lines_revisit<8, false><<<(a.n_rev[0] + 3) / 4, 128, 0, s>>>(a);
   run_walk<GL, 1, 1, 2>(a, s);
-  if (a.n_rev[1]) k_lines_revisit<true><<<(a.n_rev[1] + 3) / 4, 128, 0, s>>>(a);
+  if (a.n_rev[1]) k_lines_revisit<8, true><<<(a.n_rev[1] + 3) / 4, 128, 0, s>>>(a);
   run_walk<GL, 2, 1, 3>(a, s);
   k_lines_columns<<<(2 * a.H * (a.n / 8) + 255) / 256, 256, 0, s>>>(a);
   run_walk<GL, 3, 2, -1>(a, s);
@@ -840,10 +889,13 @@ int run_sgm_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw
   for (int i = 0; i < 4; i++) u.gw[i] = gw[i];
   launch_p2_table(u, reinterpret_cast<uint2*>(base + L.p2t), s);
   if (small_form(W, H, n)) {
-    if (n <= 32) run_small<4>(a, s);
-    else if (n <= 64) run_small<8>(a, s);
-    else if (n <= 128) run_small<16>(a, s);
-    else run_small<32>(a, s);
+    // four planes a lane up to 128: half the instructions a step of eight, for twice the warps (ms, four / eight: 520x390 D=32
+    // 0.27 / 0.29, 1431x1073 D=64 0.93 / 0.96, 1600x1200 D=128 1.85 / 2.12, 2080x1560 D=64 1.6 / 1.9, 4160x3120 D=32 3.1 / 4.2)
+    if (n <= 16) run_small<4, 4>(a, s);
+    else if (n <= 32) run_small<8, 4>(a, s);
+    else if (n <= 64) run_small<16, 4>(a, s);
+    else if (n <= 128) run_small<32, 4>(a, s);
+    else run_small<32, 8>(a, s);
   } else {
     if (n <= 64) run_large<8>(a, s);
     else if (n <= 128) run_large<16>(a, s);

@@ -89,3 +89,19 @@ def test_lines_yields_to_pass1_and_chosen_forms(ctx):
     finally:
         api.set_tuned_form(123, 77, 40, 16, 0)
     assert _solve(ctx, wl)[0] == LINES
+
+
+# the large form of four and two lines a warp, and the small form's widths of four planes a lane on either side of its limits
+@pytest.mark.parametrize("w,h,d,tile", [(2901, 2803, 64, 32), (2101, 1903, 128, 64), (1999, 1901, 128, 64), (611, 333, 16, 64), (413, 301, 24, 32),
+                                        (300, 211, 40, 16), (301, 203, 72, 64), (250, 120, 128, 8), (250, 120, 136, 8)])
+def test_lines_lane_widths_equal_chains(ctx, w, h, d, tile):
+    from lux_b200 import synth
+    wl = synth.rectified_pair(w, h, d, seed=17, tile=tile)
+    form, agg, depth = _solve(ctx, wl, keep_agg=True)
+    assert form == LINES
+    form, agg2, depth2 = _solve(ctx, wl, keep_agg=True, sgm="split")
+    assert form == 2
+    assert np.array_equal(agg, agg2)
+    assert np.array_equal(depth.view(np.uint32), depth2.view(np.uint32))
+    form, _, depth3 = _solve(ctx, wl)
+    assert form == LINES and np.array_equal(depth3.view(np.uint32), depth2.view(np.uint32))
