@@ -227,14 +227,6 @@ __global__ void __launch_bounds__(256) k_cost(const CostArgs a, const LayerGeom 
   }
 }
 
-// 1/b rounded to nearest for 2^-125 <= |b| < 2^125, as __frcp_rn without its range checks and branch: one step of Markstein's
-// correction (IBM J. Res. Dev. 34(1), 1990) from an approximation within an ulp. Compared with __frcp_rn over every mantissa.
-LUX_DEV float rcp_mid(float b) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  return __fmaf_rn(__fmaf_rn(-b, r, 1.0f), r, r);
-}
-
 // Uniform layers (every pixel searches planes [0, n), cap n, n % 8 == 0; 1 to 15 other cameras): lanes over 32
 // neighbouring pixels of a row, each walking its pixel's planes in order like the reference's loop. Eight planes at a time
 // go through camera after camera: the camera's constants, its last computed cost (:273-274, kept in shared memory between

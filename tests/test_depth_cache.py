@@ -174,3 +174,14 @@ def test_set_empty_image(api):
     with pytest.raises(O.OracleError) as e:
         O.depth_cache_set(np.ones((3, 3), np.float32), 0, 4)
     assert e.value.code == 15
+
+
+def test_fetch_every_exponent_both_reciprocals(api):
+    """Every sign, exponent and rcpps table index at the cache's own grid, in columns of the Newton pass and in the divided rest."""
+    rng = np.random.default_rng(10)
+    b = (np.arange(1 << 21, dtype=np.uint32) << 11) | rng.integers(0, 2048, 1 << 21).astype(np.uint32)
+    b = b[: (1 << 21) // 47 * 47].reshape(-1, 47)  # 32 columns by Newton, 15 by division
+    d = np.ascontiguousarray(np.concatenate([b, b[:, ::-1][:, :47]], axis=0)).view(np.float32)
+    h, w = d.shape
+    got = api.DepthImageCache.fetch(d, (0, 0, w, h), (w, h))
+    assert np.array_equal(_bits(got), _bits(O.depth_cache_fetch(d, (0, 0, w, h), (w, h))))
