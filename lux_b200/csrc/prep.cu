@@ -328,12 +328,12 @@ __global__ void __launch_bounds__(128) k_shift_resize(const uint8_t* __restrict_
                                                       int stepY, uint8_t* __restrict__ g2) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= pw) return;
-  const int sx = (int)(((long long)stepX * x) >> 16);
+  const int sx = (int)((unsigned)stepX * (unsigned)x) >> 16;  // the accumulated xAcc: an int that wraps, past 32767 columns
   int cols[4];
 #pragma unroll
   for (int j = 0; j < 4; j++) cols[j] = min(max(sx - 1 + j, 0), gw - 1);  // clamp to edge
   for (int y = blockIdx.y; y < ph; y += gridDim.y) {  // gridDim.y is capped at 65535 rows; taller images loop
-    const int sy = (int)(((long long)stepY * y) >> 16);
+    const int sy = (int)((unsigned)stepY * (unsigned)y) >> 16;
     uint32_t px[4][4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {

@@ -45,3 +45,38 @@ def test_guide_at_an_odd_address(oracle):
                                                d_out.data_ptr(), None))
     od, _ = oracle.upsample(depth, pw, ph, guide, pw, ph)
     assert np.array_equal(d_out.cpu().numpy().view(np.uint32), od.view(np.uint32))
+
+
+def _resampled_guide(guide, pw, ph):
+    """ImageShift(guide, 0.5, 0.5) at the positions of NearestResize (DenseUpsampleLayer.cs:98-131), which are sums of 32-bit
+    integers: past 32767 rows or columns they wrap below 0, where the reference reads in front of its image and this library
+    takes the first row or column."""
+    gh, gw, _ = guide.shape
+
+    def taps(n, size):
+        acc = (np.arange(n, dtype=np.int64) * int(size * 65536.0 / n)).astype(np.uint32).astype(np.int32)
+        return np.clip((acc >> 16)[:, None] - 1 + np.arange(4), 0, size - 1), acc
+    rows, ay = taps(ph, gh)
+    cols, ax = taps(pw, gw)
+    assert ay.min() < 0 or ax.min() < 0
+    k = np.array([-1, 9, 9, -1], np.int64)  # sixteenths of the half-pixel cubic taps, exact in the reference's floats
+    v = np.einsum("i,yxic->yxc", k, guide.astype(np.int64)[rows.T].transpose(1, 2, 0, 3))
+    v = np.einsum("j,yxjc->yxc", k, v[:, cols])
+    return np.clip(np.rint(v / 256.0), 0, 255).astype(np.uint8)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pw,ph", [(16500, 3), (3, 16500), (40000, 2)])
+def test_guide_positions_wrap(oracle, pw, ph):
+    from lux_b200 import api
+    rng = np.random.default_rng(pw + ph)
+    depth = rng.uniform(300.0, 6000.0, (ph, pw)).astype(np.float32)
+    guide = rng.integers(0, 256, (2 * ph, 2 * pw, 4), dtype=np.uint8)
+    g2 = np.ascontiguousarray(_resampled_guide(guide, pw, ph))
+    inv, up, want = np.empty_like(depth), np.empty((2 * ph, 2 * pw), np.float32), np.empty((2 * ph, 2 * pw), np.float32)
+    L, ptr, i32 = oracle.lib(), (lambda a: ctypes.c_void_p(a.ctypes.data)), ctypes.c_int
+    L.lo_inverse_depth(ptr(depth), ctypes.c_size_t(depth.size), ptr(inv))
+    L.lo_bilateral_upsample(ptr(inv), i32(pw), i32(ph), ptr(guide), i32(2 * pw), i32(2 * ph), i32(2 * pw), ptr(g2), ctypes.c_float(10.0), ptr(up))
+    L.lo_inverse_depth(ptr(up), ctypes.c_size_t(up.size), ptr(want))
+    r = api.DenseUpsampleLayer.run(depth, pw, ph, guide, pw, ph, sigma=10.0)
+    assert np.array_equal(r.Depth.reshape(want.shape).view(np.uint32), want.view(np.uint32))
