@@ -6,19 +6,22 @@
 // keeps the flat buffer (2 halves x (W+2) slots x (4·MaxHi+5) u16, plus Min/RangeS/RangeC/Pix) in global memory and runs
 // every Pixel() call of the reference in an order that gives each read the same last writer:
 //   * a band of T >= 4 rows runs on blocks (parts) of min(8, T/2) rows, a warp per row (one block below); blocks take
-//     tickets in order, so a part only ever waits on a running one;
+//     tickets in order, so a part only ever waits on a running one, or on a later part of its own band (at most sixteen,
+//     which start as earlier bands finish);
 //   * a part runs its tiles in order (a block barrier between tiles); inside a tile, row r runs its offset u (pixel
 //     column iT - r + u) once row r-1 has finished offset u, and a part's first row follows the part above's last row:
 //     at the same tile and offset within a band, at offset u of tile i+1 across bands (the same sheared frame);
 //   * two calls touch a common element only when at most two columns apart, and the one pair this leaves unordered,
-//     the upper row's pixel two columns right of the lower one, touches nothing in common (see the row hand-over);
+//     the upper row's pixel two columns right of the lower one, touches nothing in common unless the lower one's range
+//     reaches past the last plane, when waits of its own order the two (see the row hand-over);
 //   * the revisits of the last column do not follow the sheared columns: all of a band's revisits lie at offset 0 of its
 //     last tile, and the next band's first part waits for that offset before a tile that reaches column W-3; a part
 //     whose rows revisit in tile i first waits for the band's last part to finish tile i-1 (a band's tiles come in order
 //     in the reference);
 //   * tiles taller than the flag rows step with a block barrier instead, pixel (r, u) at step u + 2r (pixels of one step
 //     are three or more columns apart), one block per band, three tiles behind the band above.
-// tests/test_replay_schedule_cpu.py checks these waits against the reference's order as a happens-before model.
+// tests/test_replay_schedule_cpu.py and test_replay_spills_cpu.py check these waits against the reference's order as a
+// happens-before model.
 // Within a Pixel() call a warp handles the lanes, with all of the call's line-buffer reads in one batch where its windows
 // allow. The four paths run in order (a path may spill into the next), or at once on four groups of eight lanes where
 // no window of the call leaves its block.
@@ -384,6 +387,10 @@ LUX_DEV void emu_pixel(const EmuArgs& a, int x, const EmuPix& px, int cur, int o
   __syncwarp();
 }
 
+// Whether a pixel's path-3 window passes the pad after its neighbour's slot (index MaxHi + 1 of block 3), into the first
+// planes of path 0's block in the slot after that one.
+LUX_DEV bool emu_past_block(const EmuArgs& a, int start, int cap) { return start - a.min_lo + cap > a.max_hi + 1; }
+
 // The tile's pixel (row r, xp offset u) of a band: x, y and whether there is one. The clamped row start revisits the
 // last column at u = 0 only.
 struct EmuTileRow {
@@ -421,7 +428,6 @@ constexpr int kFlagRows = 64;  // tiles up to this many rows hand over row to ro
 // barrier per step of the sheared schedule, pixel (r, u) at step u + 2r (pixels of one step are three or more columns
 // apart).
 //
-//
 // Each warp owns one row of its part and runs the row's offsets u in order through all tiles; row r runs offset u of a
 // tile once row r-1 has finished offset u (a CTA-scope release/acquire of the row's count in shared memory): the
 // recurrence reads row r-1 at columns x-1, x and x+1, offsets u-2..u. For rows r1 < r2 this orders (r1, u1) before
@@ -432,7 +438,11 @@ constexpr int kFlagRows = 64;  // tiles up to this many rows hand over row to ro
 //     path-3 window, the pad element of the next slot in memory; the upper pixel writes its own blocks (never its own
 //     pad) and spills at most align - 2 <= 6 elements (q + cap <= MaxHi - MinLo + align - 1) into the pad and first
 //     block-0 elements of its next slot in memory, which is column x2 + 3 (pass +1) or x2 + 1 (pass -1), where the lower
-//     pixel reads only block 3 from index -1 (block 2's last);
+//     pixel reads only block 3 from index -1 (block 2's last). A lower pixel whose range reaches past the block (q + cap >
+//     MaxHi + 1) reads past that pad, up to element 5 of the next slot's block 0: in pass +1 the upper pixel's own. The
+//     pair is then ordered as the reference visits it: the lower pixel waits for one offset more, and at a tile's end,
+//     where the upper pixel belongs to the next tile, the upper row waits for the lower one. (In pass -1 the next slot in
+//     memory is column x2's, and paths 0 to 2 end in their own slots.);
 //   * the lower pixel writes the other half, which the upper pixel reads at columns x2+1..x2+3: its spill (pass +1)
 //     reaches slot x2+1's pad and block-0 elements 0..5, and the upper pixel reads that slot's block 1 from index -1,
 //     block 0's last element (index MaxHi >= 8 with align 8; with align 2 nothing spills).
@@ -496,8 +506,18 @@ __global__ void __launch_bounds__(kThreads) k_sgm_emulate(const EmuArgs a) {
         gneed = i * T;  // (a first part's row r0 revisiting at tile i has no tile i+2 wait: i * T >= W)
         gflag = a.progress + ((size_t)j * a.parts + last);
       }
+      // The row below comes first where its last pixel of the tile before reads past its block (see below): the slot it
+      // looks into is this row's next pixel's.
+      bool below_first = false;
+      if (a.dir > 0 && i > 0 && r + 1 < T && j * T + r + 1 < a.H && i * T - r - 2 >= 0 && i * T - r < a.W) {
+        const int pi = (j * T + r + 1) * a.W + i * T - r - 2;
+        below_first = emu_past_block(a, a.start[pi], a.cap[pi]);
+      }
       bool failed = false;
-      if (gneed > 0 && __reduce_min_sync(0xffffffffu, wait_at_least_value(gflag, gneed, a.err, 11, a.timeout_ns)) < 0) {
+      if (below_first && __any_sync(0xffffffffu, r + 1 < r1 ? !wait_shared_at_least(&s_row[r + 1], i * T, &s_stop, a.timeout_ns)
+                                                            : wait_at_least_value(a.progress + (k + 1), i * T, a.err, 11, a.timeout_ns) < 0)) {
+        failed = true;
+      } else if (gneed > 0 && __reduce_min_sync(0xffffffffu, wait_at_least_value(gflag, gneed, a.err, 11, a.timeout_ns)) < 0) {
         failed = true;
       } else if (i > 0 && i * T - r >= a.W && r != r_pub &&
                  __any_sync(0xffffffffu, !wait_shared_at_least(&s_row[r_pub], i * T, &s_stop, a.timeout_ns))) {
@@ -521,7 +541,11 @@ __global__ void __launch_bounds__(kThreads) k_sgm_emulate(const EmuArgs a) {
         // The next offset's read-only inputs, loaded while this offset waits and runs.
         has_next = u + 1 < T && emu_tile_pixel(a, row, i, r, u + 1, nx, ny);
         if (has_next) next = emu_load_pix(a, nx, ny);
-        if (r > r0 && __any_sync(0xffffffffu, !wait_shared_at_least(&s_row[r - 1], i * T + u + 1, &s_stop, a.timeout_ns))) {
+        // a pixel that reads past its block looks into the slot of the row above's next offset (but the next tile's, which
+        // the reference visits later, within a band)
+        const int more = has && a.dir > 0 && emu_past_block(a, px.start, px.cap) ? 1 : 0;
+        const int need = i * T + min(u + 1 + more, T);
+        if (r > r0 && __any_sync(0xffffffffu, !wait_shared_at_least(&s_row[r - 1], need, &s_stop, a.timeout_ns))) {
           if (lane == 0) {
             atomicCAS(a.err, 0, 11);
             s_stop = 1;
@@ -531,7 +555,7 @@ __global__ void __launch_bounds__(kThreads) k_sgm_emulate(const EmuArgs a) {
         // The first row continues the part above's last row one row down: within the band, that row at the same
         // tile and offset; across bands, the band above's last row at offset u of tile i+1 (the same sheared frame).
         if (r == r0 && k > 0) {
-          const int target = part > 0 ? i * T + u + 1 : min((i + 1) * T + u + 1, a.gwN * T);
+          const int target = part > 0 ? need : min((i + 1) * T + u + 1 + more, a.gwN * T);
           if (seen < target) {
             seen = __reduce_min_sync(0xffffffffu, wait_at_least_value(above, target, a.err, 11, a.timeout_ns));
             if (seen < 0) {
