@@ -92,6 +92,7 @@ LUX_DEV void state_new(RState& s, const RagArgs& a, uint16_t* buf, int lane) {  
   __syncwarp();
 }
 LUX_DEV void state_init(RState& s, int lane) {
+  __syncwarp();  // the copy has been read (ragged_add: a lane's planes lie in other lanes' quads)
   clear_rounds(s.cur, s.lo, s.hi, lane);
   s.lo = 1;
   s.hi = 0;
@@ -201,7 +202,7 @@ LUX_DEV void edge_start(const RagArgs& a, int p, int x, RState& s, uint32_t& P2,
   P2 = p2_between(a, x, a.H - 1, xe, a.y_b);
 }
 
-// Per batch and lane i (mod 8): pixel i's aggregate offset / 8, its range and the P2 of the path in hand.
+// Per batch and lane i (mod kBatch): pixel i's aggregate offset / 8, its range and the P2 of the path in hand.
 struct Px {
   uint32_t off8, qc, p2;
 };
@@ -241,7 +242,7 @@ LUX_DEV void ragged_chain(const RagArgs& a, int x, int lane, uint8_t* ring, RSta
   const int K = T - (W - 1) % T, full = T + K, tail = H % T;
   const int steps = (H / T) * full + (tail ? tail + min(K, tail) : 0);
   auto pix = [&](int t) { return (BWD ? H - 1 - t : t) * W + x; };
-  auto load_row = [&](int b) {  // lane i (mod 8): step i's row of the pass; bit 29: a revisit, bit 30: a band's first one
+  auto load_row = [&](int b) {  // lane i (mod kBatch): step i's row of the pass; bit 29: a revisit, bit 30: a band's first one
     const int s = min(b * kBatch + (lane & (kBatch - 1)), steps - 1);
     const int j = s / full, o = s - j * full, base = j * T, v = min(K, min(T, H - base));
     return (o < v ? base + o : base + o - v) | (o >= v && o < 2 * v ? 1 << 29 : 0) | (o == v ? 1 << 30 : 0);
@@ -271,6 +272,7 @@ LUX_DEV void ragged_chain(const RagArgs& a, int x, int lane, uint8_t* ring, RSta
       if (ev & (1 << 30)) {
         const int v = min(K, min(T, H - t)), src = (v & 1) ? t + v - 2 : t + v - 1;
         if ((v & 1) && src >= 0) {
+          __syncwarp();  // the copy that the next step writes has been read
           s.flip();
           s.md = md_before;
         }
