@@ -277,6 +277,7 @@ LUX_DEV void column_chain(const LineArgs& a, int x, int lane, typename RawOf<K>:
       }
     }
     const int rv2 = load_rows(b + 2);
+    __syncwarp();  // every lane has read the batch's costs before they are replaced
     if (b + 2 < nb) stage(b + 2, rv2);
     else cp_async_commit();
     rv = rvn;
