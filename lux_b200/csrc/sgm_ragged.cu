@@ -307,6 +307,8 @@ LUX_DEV void ragged_chain(const RagArgs& a, int x, int lane, uint8_t* ring, RSta
   cp_async_wait<0>();
 }
 
+// A pixel's ring slot: a range is at most MaxHi + 7 long; a quad may read a word past it.
+constexpr int ring_bytes_of(int max_hi) { return (kPad + max_hi + 8 + 8 + 15) & ~15; }
 __host__ __device__ constexpr int warp_smem(int rounds, int ring_bytes) { return 2 * kBatch * ring_bytes + ((2 * state_u16(rounds) * 2 + 15) & ~15); }
 
 // The four paths of a pass, a warp a line; warp 0 takes the special column's path 2.
@@ -527,15 +529,15 @@ int run_ragged_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float
   for (int i = 0; i < 4; i++) a.gw[i] = gw[i];
   a.edge = reinterpret_cast<uint16_t*>(base + L.edge);
   a.edge_min = reinterpret_cast<uint16_t*>(base + L.edge_min);
-  a.ring_bytes = (kPad + g.max_hi + 8 + 8 + 15) & ~15;  // a range is at most MaxHi + 7 long; a quad may read a word past it
+  a.ring_bytes = ring_bytes_of(g.max_hi);
   uint4* info = reinterpret_cast<uint4*>(base + L.info);
   a.info = info;
   k_ragged_info<<<(W * H + 255) / 256, 256, 0, s>>>(a, g.start, g.cap, g.off, g.min_lo, info);
   count_launches(1);
   a.rounds = rounds_of(g.max_hi);
   const int blocks = (1 + 3 * W + H + 1) / 2, smem = 2 * warp_smem(a.rounds, a.ring_bytes);
-  for (auto k : {k_ragged_pass<false>, k_ragged_pass<true>, k_ragged_revisit<false>, k_ragged_revisit<true>})
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // (a kernel's limit is one for all threads of the process: another one's smaller layer must not lower it before this launch)
+  static_assert(2 * warp_smem(kMaxRounds, ring_bytes_of(kMaxRounds * kRound - 9)) <= 48 * 1024, "within every kernel's default limit");
   k_ragged_pass<false><<<blocks, 64, smem, s>>>(a);
   if (a.n_rev[0]) k_ragged_revisit<false><<<(a.n_rev[0] + 1) / 2, 64, smem, s>>>(a);
   k_ragged_pass<true><<<blocks, 64, smem, s>>>(a);
