@@ -18,6 +18,7 @@
 // revisit batches in the reference's order; path 3 restarts from the margin.
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -683,10 +684,14 @@ void launch_chains_t(const SplitArgs& a, cudaStream_t s) {
   cudaMemsetAsync(a.bnd, 0, entries * Dp_of(LPT) * 2, s);
   cudaMemsetAsync(a.bnd_min, 0, entries * 2, s);
   const size_t smem = chain_smem_bytes<LPT>(nw, a.u.n, PASS2 || GROUP == 1);
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaFuncSetAttribute(k_chains<LPT, FULL, PASS2, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    configured = smem;
+  {
+    static std::mutex mu;  // the kernel's limit is the process's: it only grows, whichever threads launch
+    static size_t configured = 0;
+    std::lock_guard<std::mutex> lk(mu);
+    if (smem > configured) {
+      cudaFuncSetAttribute(k_chains<LPT, FULL, PASS2, GROUP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      configured = smem;
+    }
   }
   k_chains<LPT, FULL, PASS2, GROUP><<<chain_blocks(a.nchains), (nw + 2) * 32, smem, s>>>(a);
   count_launches(1);
