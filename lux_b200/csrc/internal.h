@@ -194,9 +194,10 @@ int run_sgm_wave(const LayerGeom& g, int xsw, uint16_t p1, float p2scale, const 
 // sgm_lines.cu: the same aggregation one path at a time along independent lines (n <= 256; pass +1's aggregates never exist
 // by themselves, so it cannot keep them)
 bool lines_supported(int W, int n);
-size_t lines_scratch_bytes(int W, int H, int n);
+bool lines_keep_states(int W, int H, int n);  // the size rule between its two variants: with kept states (half the raw costs' bytes more) or without
+size_t lines_scratch_bytes(int W, int H, int n, bool keep_states);
 int run_sgm_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg, float* depth,
-                  int keep_agg, void* scratch, size_t scratch_bytes, cudaStream_t s);
+                  int keep_agg, bool keep_states, void* scratch, size_t scratch_bytes, cudaStream_t s);
 // sgm_ragged.cu: the same for ragged layers and uniform ones past 256 planes. *flag (device) becomes 1 where the layer's ranges
 // meet the ends of the reference's line buffer in a way that only the exact replay follows.
 void launch_ragged_check(const LayerGeom& g, int* flag, cudaStream_t s);

@@ -401,10 +401,13 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     ca.unit = Wm[0] == Wm[10] && Wm[5] == Wm[10] && Wm[14] == 0.0f && Wm[10] != 0.0f && ca.norm_mul ? 1 : 0;
   }
   const size_t phase_words = ca.vcols ? 8 : 4;  // per pixel: four phases of a word, or of the vertical triples' u16 pairs
-  for (int k = 0; k < ca.n_others; k++) {  // the half-pixel phase images of the other cameras
-    uint32_t* ph = nullptr;
-    const size_t words = ca.unit ? cost_unit_phase_bytes(ca.ow[k], ca.oh[k], L->n) / 4 : phase_words * ca.ow[k] * ca.oh[k];
-    if ((rc = alloc_t(ctx, phases, words, &ph))) return rc;
+  // the half-pixel phase images of the other cameras; where the byte images (padded columns: narrow images take more than
+  // the triples) find no memory, the triples are used
+  uint32_t* ph = nullptr;
+  if (ca.unit && alloc_quiet(ctx, phases, cost_unit_phase_bytes(ca.ow[0], ca.oh[0], L->n) / 4, &ph)) ca.unit = 0;
+  ca.phase[0] = ph;
+  for (int k = 0; k < ca.n_others && !ca.unit; k++) {
+    if ((rc = alloc_t(ctx, phases, phase_words * ca.ow[k] * ca.oh[k], &ph))) return rc;
     ca.phase[k] = ph;
   }
   CK(cudaEventRecord(ctx->ev[0], s));
@@ -414,10 +417,11 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
   // aggregation: two passes over the sheared tiles, then WTA
   CK(cudaEventRecord(ctx->ev[1], s));
   const int xsw = 0;  // LUX_SGM_XSW unset: the reference default (DenseStereoSgm.cs:31)
-  if (ragged_lines) {
-    void* scr = nullptr;
-    const size_t sb = ragged_lines_scratch_bytes(W, H, L->max_hi);
-    if ((rc = dev_alloc(ctx, tmp, sb, &scr))) return rc;
+  char* lines_scr = nullptr;  // the lines' tables and states: where they find no memory, the form that ran before them does
+  const size_t ragged_sb = ragged_lines ? ragged_lines_scratch_bytes(W, H, L->max_hi) : 0;
+  if (ragged_lines && alloc_quiet(ctx, tmp, ragged_sb, &lines_scr) == LUX_OK) {
+    void* scr = lines_scr;
+    const size_t sb = ragged_sb;
     if ((rc = run_ragged_lines(g, p.p1, p.p2scale, p.guidance, L->raw, L->agg, scr, sb, s)))
       return set_err(ctx, LUX_ERR_CUDA, "ragged aggregation launch failed (%d)", rc);
     CK(cudaEventRecord(ctx->ev[2], s));
@@ -437,14 +441,20 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     const bool wide = uniform_wide_planes(L->n);
     const int forced = wide ? 1 : (flags & LUX_LAYER_SGM_WAVE) ? 3 : (flags & LUX_LAYER_SGM_SPLIT) ? 2 : (flags & LUX_LAYER_SGM_FUSED) ? 1 : 0;
     int form = forced;
-    bool tune = false;
+    bool tune = false, keep_states = false;
     if (!forced) {
       const TunedForm t = tuned_form(W, H, L->n, p.tile);
       // The lines form is faster than the other three at every size (4160x3120 D=256: 15.4 against 17.6 ms; 1040x780
       // D=64: 0.64 against 4.5 ms; 520x390 D=32: 0.26 against 2.4 ms) but never holds pass +1's aggregates alone and waits on nothing (debug_stall).
       if (!(flags & LUX_LAYER_KEEP_PASS1) && !t.set_by_caller && ctx->stall_block < 0 && lines_supported(W, L->n)) {
-        form = 4;
-      } else {
+        keep_states = lines_keep_states(W, H, L->n);
+        if (alloc_quiet(ctx, tmp, lines_scratch_bytes(W, H, L->n, keep_states), &lines_scr) == LUX_OK) form = 4;
+        else if (keep_states && alloc_quiet(ctx, tmp, lines_scratch_bytes(W, H, L->n, false), &lines_scr) == LUX_OK) {
+          form = 4;
+          keep_states = false;  // slower at this size, in far less memory
+        }
+      }
+      if (form == 0) {
         form = t.form;
         tune = form == 0 && ctx->autotune;
         if (form == 0) form = (size_t)W * H >= 2000000 ? 2 : 1;  // untuned: the path-group chains from about 2 MP
@@ -452,10 +462,10 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     }
     const int keep = (flags & LUX_LAYER_KEEP_AGG) ? 1 : 0;
     auto scratch_of = [&](int f) {
-      return f == 4 ? lines_scratch_bytes(W, H, L->n) : f == 2 ? split_scratch_bytes(W, H, L->n) : f == 3 ? wave_scratch_bytes(W, H, L->n) : uniform_scratch_bytes(W, H, L->n, p.tile);
+      return f == 4 ? lines_scratch_bytes(W, H, L->n, keep_states) : f == 2 ? split_scratch_bytes(W, H, L->n) : f == 3 ? wave_scratch_bytes(W, H, L->n) : uniform_scratch_bytes(W, H, L->n, p.tile);
     };
     auto run_form = [&](int f, void* scr, size_t sb) {
-      if (f == 4) return run_sgm_lines(g, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->depth, keep, scr, sb, s);
+      if (f == 4) return run_sgm_lines(g, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->depth, keep, keep_states, scr, sb, s);
       if (f == 2) return run_sgm_split(g, xsw, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->agg_pass1, L->depth, keep, scr, sb, ctx->d_err, s);
       if (f == 3) return run_sgm_wave(g, xsw, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->agg_pass1, L->depth, keep, scr, sb, ctx->d_err, s);
       return run_sgm_uniform(g, xsw, p.p1, p.p2scale, p.guidance, L->raw, L->agg, L->agg_pass1, L->depth, keep, scr, sb, ctx->d_err, s);
@@ -497,9 +507,9 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
       L->tuned = best;
       return LUX_OK;
     }
-    void* scr = nullptr;
+    void* scr = lines_scr;
     const size_t sb = scratch_of(form);
-    if ((rc = dev_alloc(ctx, tmp, sb, &scr))) return rc;
+    if (form != 4 && (rc = dev_alloc(ctx, tmp, sb, &scr))) return rc;
     if ((rc = run_form(form, scr, sb))) return set_err(ctx, LUX_ERR_CUDA, "uniform aggregation launch failed (%d)", rc);
     CK(cudaEventRecord(ctx->ev[2], s));
     CK(cudaEventRecord(ctx->ev[3], s));

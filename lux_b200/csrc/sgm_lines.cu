@@ -13,7 +13,7 @@
 // cycles of a scheduler (44.3 without its loads; 53.7 with pairs of adjacent planes, 62 with the DPX min/add forms): the
 // 16-bit minima and permutes bound it, so the adds are multiply-adds by a kernel-argument one, which issue elsewhere. A
 // line takes GL = 4, 8, 16 or 32 lanes (planes / K, rounded
-// up to a power of two), so a warp carries 32 / GL neighbouring lines. Two forms, chosen by size (run_sgm_lines):
+// up to a power of two), so a warp carries 32 / GL neighbouring lines. Two variants, chosen by size (small_form):
 //   * small layers: the four paths of a pass in one launch, each adding its L into the aggregates by reductions in L2 (four
 //     u16 sums in a 64-bit add, none of which can carry). A pass is as long as one line: latency is what such a layer costs.
 //   * large layers, path by path: k_lines_ckpt walks the lines forward and keeps the path's state every kSeg pixels;
@@ -771,12 +771,12 @@ bool small_form(int W, int H, int n) {
   return W < 2 * kSeg || n <= 32 || (size_t)W * H * n < (size_t)(n <= 128 ? 480 : 240) << 20;
 }
 
-LinesLayout lines_layout(int W, int H, int n) {
+LinesLayout lines_layout(int W, int H, int n, bool keep_states) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   LinesLayout s;
   size_t o = 0;
   // states: W + 1 lines or fewer of at most H + H / (W - 1) + 1 steps, or H lines of W
-  const size_t states = small_form(W, H, n) ? 0 : std::max((size_t)(W + 1) * ((H + H / (W - 1) + 1) / kSeg + 1), (size_t)H * (W / kSeg + 1));
+  const size_t states = !keep_states ? 0 : std::max((size_t)(W + 1) * ((H + H / (W - 1) + 1) / kSeg + 1), (size_t)H * (W / kSeg + 1));
   for (int k = 0; k < 2; k++) {
     s.ckpt[k] = o; o += al(states * n * 2);
     s.ckpt_min[k] = o; o += al(states * 2);
@@ -837,15 +837,16 @@ void run_large(const LineArgs& a, cudaStream_t s) {
 // The layers this form takes, beyond uniform_fast_supported's: at most 256 planes, and rows of a batch's length or more (a
 // diagonal wraps at most once in a batch).
 bool lines_supported(int W, int n) { return n <= kState && W >= kBatch; }
-size_t lines_scratch_bytes(int W, int H, int n) { return lines_layout(W, H, n).total; }
+bool lines_keep_states(int W, int H, int n) { return !small_form(W, H, n); }
+size_t lines_scratch_bytes(int W, int H, int n, bool keep_states) { return lines_layout(W, H, n, keep_states).total; }
 
 // k_p2_table lives in sgm_uniform.cu
 void launch_p2_table(const UniArgs& a, uint2* p2t, cudaStream_t s);
 
 int run_sgm_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw[4], const uint8_t* raw, uint16_t* agg, float* depth,
-                  int keep_agg, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+                  int keep_agg, bool keep_states, void* scratch, size_t scratch_bytes, cudaStream_t s) {
   const int W = g.W, H = g.H, n = g.n_planes, T = g.tile;
-  const LinesLayout L = lines_layout(W, H, n);
+  const LinesLayout L = lines_layout(W, H, n, keep_states);
   if (scratch_bytes < L.total) return 9;
   char* base = static_cast<char*>(scratch);
   LineArgs a;
@@ -889,7 +890,7 @@ int run_sgm_lines(const LayerGeom& g, uint16_t p1, float p2scale, const float gw
   u.W = W; u.H = H; u.dir = 1; u.guidance = g.guidance; u.p2base = a.p2base; u.y_b = -1;
   for (int i = 0; i < 4; i++) u.gw[i] = gw[i];
   launch_p2_table(u, reinterpret_cast<uint2*>(base + L.p2t), s);
-  if (small_form(W, H, n)) {
+  if (!keep_states) {
     // four planes a lane up to 128: half the instructions a step of eight, for twice the warps (ms, four / eight: 520x390 D=32
     // 0.27 / 0.29, 1431x1073 D=64 0.93 / 0.96, 1600x1200 D=128 1.85 / 2.12, 2080x1560 D=64 1.6 / 1.9, 4160x3120 D=32 3.1 / 4.2)
     if (n <= 16) run_small<4, 4>(a, s);
