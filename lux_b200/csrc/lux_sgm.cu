@@ -215,6 +215,8 @@ lux_stereo_params default_params() {
   return p;
 }
 
+constexpr size_t kMaxReplayElems = (size_t)INT_MAX - 65536;  // the replay indexes its line buffer with 32-bit integers
+
 struct RangeResult {
   int min_lo, max_hi_raw;
 };
@@ -323,6 +325,8 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
                          (uniform ? LUX_LAYER_SGM_FUSED | LUX_LAYER_SGM_SPLIT | LUX_LAYER_SGM_WAVE : 0);
   const bool ragged_lines = !(flags & form_flags) && ctx->stall_block < 0 && !needs_replay &&
                             (!uniform || (fast && uniform_wide_planes(L->n) && !tuned_form(W, H, L->n, p.tile).set_by_caller)) &&
+                            // (a ragged layer whose line buffer the replay refuses is refused: it may hold ranges that only the replay follows)
+                            (uniform || emu_line_buffer_elems(W, L->max_hi) <= kMaxReplayElems) &&
                             ragged_lines_supported(W, H, p.tile, p.p1, p.p2scale, L->max_hi, L->volume);
   if (!fast || ragged_lines) CK(cudaMemsetAsync(L->agg, 0, (L->volume + 8) * 2, s));
   if (!uniform) CK(cudaMemsetAsync(L->raw, 0, L->volume + 8, s));
@@ -526,7 +530,7 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
   const int bands = (H + p.tile - 1) / p.tile;
   EmuBuffers eb;
   eb.Llen = emu_line_buffer_elems(W, L->max_hi);
-  if (eb.Llen > (size_t)INT_MAX - 65536)  // the replay indexes its line buffer with 32-bit integers
+  if (eb.Llen > kMaxReplayElems)
     return set_err(ctx, LUX_ERR_UNSUPPORTED, "the exact replay's line buffer of %zu elements is past 32-bit indexing", eb.Llen);
   if ((rc = alloc_t(ctx, tmp, eb.Llen, &eb.L))) return rc;
   if ((rc = alloc_t(ctx, tmp, (size_t)2 * (W + 2) * 4, &eb.Min))) return rc;
