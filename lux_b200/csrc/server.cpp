@@ -12,6 +12,7 @@
 // planes, schedules) of the others. A request is one layer solved exactly as lux_sgm_layer solves it (prefilter
 // included), its depth map read back into the caller's host buffer; the server adds no arithmetic of its own, so every
 // result equals the same request run alone.
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -23,6 +24,7 @@
 #include <vector>
 
 #include "../../include/lux_sgm.h"
+#include "internal.h"
 
 namespace {
 
@@ -73,8 +75,10 @@ struct lux_server {
 namespace {
 
 // Device bytes a request needs, estimated from its sizes: the cost volume and aggregates of its layer (volume = pixels x
-// planes, 3 bytes each, plus 2 per kept aggregate set), per-pixel tables and the aggregation scratch (about 100 bytes a
-// pixel), the filtered images and half-pixel phase images (40 bytes a pixel per camera), and 64 MiB of slack.
+// planes, 3 bytes each, plus 2 per kept aggregate set), per-pixel tables and the other forms' scratch (about 100 bytes a
+// pixel), the images and filtered images (8 bytes a pixel per camera), the larger of what is there one after the other, the
+// half-pixel phase images of the cost (32 bytes a pixel per camera) and the tables and kept states of the lines, and 64 MiB
+// of slack.
 uint64_t estimate_bytes(const Pending& p) {
   const int sc = p.params.scale > 0 ? p.params.scale : 1;
   const uint64_t W = (uint64_t)((p.images[0].w + sc - 1) / sc), H = (uint64_t)((p.images[0].h + sc - 1) / sc);
@@ -86,8 +90,11 @@ uint64_t estimate_bytes(const Pending& p) {
   const uint64_t vol = W * H * (uint64_t)n;
   uint64_t b = vol * 3 + W * H * 100 + (64ull << 20);
   if (p.flags & LUX_LAYER_KEEP_PASS1) b += vol * 2;
-  for (const auto& im : p.images) b += (uint64_t)im.w * im.h * 40;
-  return b;
+  uint64_t image_px = 0;
+  for (const auto& im : p.images) image_px += (uint64_t)im.w * im.h;
+  const int w = (int)W, h = (int)H;
+  const uint64_t lines = lux::lines_supported(w, n) ? lux::lines_scratch_bytes(w, h, n, lux::lines_keep_states(w, h, n)) : 0;
+  return b + image_px * 8 + std::max(image_px * 32, lines);
 }
 
 // The request a free worker starts (JobQueue.Dispatch, JobQueue.cs:496-521): the queue is kept in (priority, arrival)
@@ -130,12 +137,12 @@ void worker(lux_server* s, lux_sgm_ctx* ctx) {
     p.started = Clock::now();
     lux_result r{};
     lux_layer* L = nullptr;
-    // The aggregation form by size (path-group chains from about 2 MP, the fused wavefront below), unless the request
-    // names one: the autotuner's choices are timed on an idle GPU, and beside other requests they need not be the best
-    // (measured in the 60/s mixed stream: the lean wavefront for the 520x390 previews, their solo choice, gave a served
-    // p99 of 441 ms, the fused wavefront 181 ms).
+    // A request that names no form takes what a plain call takes: the lines, which no autotuner chooses and which wait on
+    // nothing, so that they suit a shared GPU as they suit an idle one. Only a request that keeps pass +1's aggregates, which
+    // the lines never hold, takes its form by size (path-group chains from about 2 MP, the fused wavefront below): the
+    // autotuner's choices are timed on an idle GPU, and beside other requests they need not be the best.
     int32_t flags = p.flags | LUX_LAYER_PREFILTER;
-    if (!(flags & (LUX_LAYER_SGM_FUSED | LUX_LAYER_SGM_SPLIT | LUX_LAYER_SGM_WAVE))) {
+    if ((flags & LUX_LAYER_KEEP_PASS1) && !(flags & (LUX_LAYER_SGM_FUSED | LUX_LAYER_SGM_SPLIT | LUX_LAYER_SGM_WAVE))) {
       const int sc = p.params.scale > 0 ? p.params.scale : 1;
       const int64_t w = (p.images[0].w + sc - 1) / sc, h = (p.images[0].h + sc - 1) / sc;
       flags |= w * h >= 2000000 ? LUX_LAYER_SGM_SPLIT : LUX_LAYER_SGM_FUSED;

@@ -165,3 +165,50 @@ def test_cancel_before_start():
             continue
         assert res[k].status == 0
         assert np.array_equal(res[k].Depth.view(np.uint32), solo[k].view(np.uint32)), k
+
+
+@pytest.mark.parametrize("keep_pass1", [False, True])
+def test_served_request_takes_the_plain_form(keep_pass1):
+    """A request that names no form launches what a plain call launches (the lines); one that keeps pass +1's aggregates takes
+    its form by size."""
+    from lux_b200 import _lib, api
+    images, gray, calibs, near, far, params = _requests()[2]
+    ctx = api.Context(0)
+    srv = api.Server(0, slots=1)
+    try:
+        def plain(**kw):
+            n = api.kernel_launches()
+            L = api.DenseLayer.compute(images, gray, calibs, near, far, params, prefilter=True, keep_pass1=keep_pass1, ctx=ctx, **kw)
+            form = L.sgm_kernel
+            L.close()
+            return form, api.kernel_launches() - n
+        form, launches = plain(sgm="fused") if keep_pass1 else plain()
+        assert form == (1 if keep_pass1 else 4)
+        n = api.kernel_launches()
+        flags = _lib.LAYER_KEEP_PASS1 if keep_pass1 else 0
+        assert srv.wait(srv.submit(images, gray, calibs, near, far, params, flags=flags)).status == 0
+        assert api.kernel_launches() - n == launches
+    finally:
+        srv.close()
+        ctx.close()
+
+
+def test_estimate_covers_the_lines_states():
+    """A pair whose second image is small: the lines' kept states are then larger than the phase images they follow."""
+    from lux_b200 import api, synth
+    wl = synth.rectified_pair(2080, 1560, 256, seed=91, bits=12, tile=64)
+    images = [wl.images[0], np.ascontiguousarray(wl.images[1][:64, :64])]
+    r = (images, wl.gray, wl.calibs, wl.near, wl.far, wl.params)
+    ctx = api.Context(0)
+    try:
+        ctx.check(ctx.lib.lux_sgm_sync(ctx.handle))
+        api.pool_high_water(0, reset=True)
+        base = api.pool_high_water(0)
+        L = api.DenseLayer.compute(*r, prefilter=True, ctx=ctx)
+        assert L.sgm_kernel == 4
+        L.close()
+        ctx.check(ctx.lib.lux_sgm_sync(ctx.handle))
+        peak = api.pool_high_water(0) - base
+        assert peak > 0 and api.Server.estimate(*r) >= peak, (api.Server.estimate(*r), peak)
+    finally:
+        ctx.close()
