@@ -479,6 +479,19 @@ struct Bilateral {
   uint64_t minus0;  // for mul_alone
 };
 
+// Every output pixel by itself, of the depth and the confidence or one of them: guides that are not word-aligned, and images
+// too small for the quads.
+template <bool DEPTH, bool CONF>
+__global__ void __launch_bounds__(128) k_bilateral_pixels(const Bilateral b) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= b.W) return;
+  for (int y = blockIdx.y; y < b.H; y += gridDim.y) {  // gridDim.y is capped at 65535 rows; taller images loop
+    const size_t at = (size_t)y * b.W + x;
+    if (DEPTH) b.out[at] = bilateral_pixel(b.prev, b.lw, b.lh, b.guide, b.gstride, b.g2, b.k, true, b.rcp, x, y);
+    if (CONF) b.out_conf[at] = bilateral_pixel(b.conf, b.lw, b.lh, b.guide, b.gstride, b.g2, b.k, false, b.rcp, x, y);
+  }
+}
+
 // The output pixels outside the quads, one by one: row 0 and the rows past the quads, then column 0 and the columns past
 // them.
 __global__ void k_bilateral_border(const Bilateral b) {
@@ -593,16 +606,24 @@ void launch_upsample(const float* prev, int pw, int ph, const uint8_t* guide, in
   const bool quads = words && b.k > 0.0f && b.k <= 3.4e38f && gw < (1 << 23) && gh < (1 << 23) && (size_t)pw * ph < ((size_t)1 << 31);
   b.qx = quads ? std::max(0, std::min((gw - 1) / 2, pw - 1)) : 0;
   b.qy = quads ? std::max(0, std::min((gh - 1) / 2, ph - 1)) : 0;
-  if (b.qx == 0 || b.qy == 0) b.qx = b.qy = 0;
-  int launches = 1;
-  if (b.qx > 0) {
+  int launches = 2;
+  // Below 150,000 quads, or 30,000 with confidence, the table's way into shared memory and the border's launch cost more than
+  // they save (us a call, quads / pixels: 260x195 25 / 21, 400x300 27.1 / 26.4, 520x390 29 / 33; with confidence 130x98 25 / 24,
+  // 200x150 25 / 25, 260x195 25 / 28).
+  if ((size_t)b.qx * b.qy < (b.conf ? 30000 : 150000)) {
+    const dim3 grid((gw + 127) / 128, std::min(gh, 65535));
+    if (!b.conf) k_bilateral_pixels<true, false><<<grid, 128, 0, s>>>(b);
+    else if (!words) k_bilateral_pixels<true, true><<<grid, 128, 0, s>>>(b);
+    else {  // (three launches, as every aligned upsample with confidence)
+      k_bilateral_pixels<true, false><<<grid, 128, 0, s>>>(b);
+      k_bilateral_pixels<false, true><<<grid, 128, 0, s>>>(b);
+      launches++;
+    }
+  } else {
     const unsigned grid = (unsigned)std::min<size_t>(((size_t)b.qx * b.qy + 255) / 256, 148 * kQuadBlocks);
     if (b.conf) k_bilateral_quads<true><<<grid, 256, 0, s>>>(b);
     else k_bilateral_quads<false><<<grid, 256, 0, s>>>(b);
-    launches++;
-  }
-  const size_t rest = (size_t)(gh - 2 * b.qy) * gw + (size_t)(gw - 2 * b.qx) * 2 * b.qy;
-  if (rest > 0) {
+    const size_t rest = (size_t)(gh - 2 * b.qy) * gw + (size_t)(gw - 2 * b.qx) * 2 * b.qy;  // row 0 at least
     k_bilateral_border<<<(unsigned)std::min<size_t>((rest + 127) / 128, 148 * 64), 128, 0, s>>>(b);
     launches++;
   }

@@ -80,3 +80,28 @@ def test_guide_positions_wrap(oracle, pw, ph):
     L.lo_inverse_depth(ptr(up), ctypes.c_size_t(up.size), ptr(want))
     r = api.DenseUpsampleLayer.run(depth, pw, ph, guide, pw, ph, sigma=10.0)
     assert np.array_equal(r.Depth.reshape(want.shape).view(np.uint32), want.view(np.uint32))
+
+
+# images past the size rule of the quads (the smaller ones above go pixel by pixel): sides of no round size, one of few rows or columns
+@pytest.mark.gpu
+@pytest.mark.parametrize("pw,ph,with_conf,sigma", [(389, 391, True, 10.0), (389, 391, False, 0.5), (16000, 11, True, 1e-3), (11, 16000, False, 300.0),
+                                                   (521, 390, True, 1e10), (521, 390, True, 1e-25)])
+def test_many_quads(oracle, pw, ph, with_conf, sigma):
+    from lux_b200 import api
+    rng = np.random.default_rng(pw + ph)
+    depth = rng.uniform(300.0, 6000.0, (ph, pw)).astype(np.float32)
+    special = np.array([0.0, -0.0, np.inf, -np.inf, 1e-40, 3e38, -5.0], np.float32)
+    depth.reshape(-1)[::7] = np.resize(special, depth.reshape(-1)[::7].size)
+    guide = rng.integers(0, 256, (2 * ph, 2 * pw, 4), dtype=np.uint8)
+    guide[: ph // 2] = 255
+    guide[ph // 2: ph] = rng.integers(0, 2, guide[ph // 2: ph].shape) * 255
+    conf = rng.uniform(0, 1, (ph, pw)).astype(np.float32) if with_conf else None
+    n0 = api.kernel_launches()
+    r = api.DenseUpsampleLayer.run(depth, pw, ph, guide, pw, ph, sigma=sigma, prev_confidence=conf)
+    assert api.kernel_launches() - n0 == 3  # resampling, quads and border (an infinite k: depth and confidence pixel by pixel)
+    od, oc = oracle.upsample(depth, pw, ph, guide, pw, ph, sigma=sigma, prev_conf=conf)
+    got = r.Depth.reshape(od.shape)
+    assert ((got.view(np.uint32) == od.view(np.uint32)) | (np.isnan(od) & np.isnan(got))).all()
+    if with_conf:
+        gc = r.Confidence.reshape(oc.shape)
+        assert ((gc.view(np.uint32) == oc.view(np.uint32)) | (np.isnan(oc) & np.isnan(gc))).all()
