@@ -644,7 +644,8 @@ void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h
   const int tiles_h = (w + kHamTile - 1) / kHamTile;
   k_hamming<LPT><<<dim3((unsigned)tiles_h * h, n), 256, 0, s>>>(cl, ps, w, h, tiles_h);
   count_launches(1);
-  if (sc.ckpt) {
+  const bool lines = sc.ckpt && census_lines_supported(w, h, 32 * LPT);
+  if (lines) {
     CensusLines a{};
     a.W = w;
     a.H = h;
@@ -681,7 +682,7 @@ void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h
   if (lr) {
     const int tiles = (w + kRight - 1) / kRight;
     const dim3 right((unsigned)tiles * h, n);
-    if (sc.ckpt) k_census_wta_right<LPT, true><<<right, kRight, 0, s>>>(ps, w, h, tiles);
+    if (lines) k_census_wta_right<LPT, true><<<right, kRight, 0, s>>>(ps, w, h, tiles);
     else k_census_wta_right<LPT, false><<<right, kRight, 0, s>>>(ps, w, h, tiles);
     k_census_lr<<<dim3((npx + 255) / 256, n), 256, 0, s>>>(ps, w, h, max_diff);
     count_launches(2);
@@ -694,7 +695,11 @@ void batch_stages(const uint64_t* cl, const CensusPairs& ps, int n, int w, int h
 size_t census_states(int w, int h) {
   return std::max((size_t)(w + 1) * ((h + h / (w - 1) + 1) / kSeg + 1), (size_t)h * (w / kSeg + 1));
 }
-bool census_lines_supported(int w) { return w >= kBatch; }
+// The lines walk each path but the first down the whole image, whatever its width; a scanline of a diagonal is as short as
+// the shorter side. Tall images of few columns have too few lines to hide that (ms, lines / scanlines: D=64 16x2000 2.8 / 1.6,
+// 64x1000 1.5 / 1.2, 100x1000 1.8 / 1.6, 200x800 1.8 / 1.8, 400x1000 3.1 / 3.7; past 64 disparities 64x5000 D=128 6.9 / 7.8,
+// 16x2000 D=256 2.3 / 1.9).
+bool census_lines_supported(int w, int h, int D) { return w >= kBatch && h <= (D <= 64 ? 3 : 80) * (long long)w; }
 int census_lpt(int D) { return D <= 32 ? 1 : D <= 64 ? 2 : D <= 128 ? 4 : D <= 256 ? 8 : 0; }
 
 void launch_census_batch(const uint8_t* ref, const uint8_t* const* others, int n, int w, int h, int stride, int bpp, uint32_t P1,

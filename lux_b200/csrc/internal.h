@@ -123,7 +123,7 @@ struct CensusScratch {
   uint16_t *ckpt, *ckpt_min;
   int pairs;
 };
-bool census_lines_supported(int w);      // the widths that the lines take
+bool census_lines_supported(int w, int h, int D);  // the images that the lines take (by the lane width of D)
 size_t census_states(int w, int h);      // kept states of a path: each of 32·census_lpt(D) values and a minimum, twice a pair
 // n pairs (<= kMaxFusePairs) of the reference image against others[k] (device pointers), all W x H; grey at byte 0 of
 // every bpp bytes, rows stride pixels apart; pair k's buffers are laid out with 32·census_lpt(D_k) values a pixel; cl:

@@ -1272,9 +1272,10 @@ int census_batch(lux_sgm_ctx* ctx, std::vector<DevBuf>& tmp, int n, const lux_im
   // Where the memory or the context's budget does not have them, the scanlines are walked without.
   CensusScratch sc{};
   std::vector<DevBuf> states;
-  if (census_lines_supported(w)) {
-    size_t Dp = 0;
-    for (int k = 0; k < n; k++) Dp = std::max(Dp, 32 * (size_t)census_lpt(Ds[k]));
+  size_t Dp = 0;  // the widest of the pairs that take the lines
+  for (int k = 0; k < n; k++)
+    if (census_lines_supported(w, h, Ds[k])) Dp = std::max(Dp, 32 * (size_t)census_lpt(Ds[k]));
+  if (Dp) {
     const size_t per = 2 * census_states(w, h);
     sc.pairs = (int)std::min<size_t>(n, std::max<size_t>(1, ((size_t)2 << 30) / (per * (Dp + 1) * 2)));
     if (alloc_quiet(ctx, states, per * sc.pairs * Dp, &sc.ckpt) || alloc_quiet(ctx, states, per * sc.pairs, &sc.ckpt_min)) sc.ckpt = nullptr;

@@ -42,3 +42,26 @@ def test_without_room_for_states():
     finally:
         ctx.close()
     assert np.array_equal(got.view(np.uint32), C.census_sgm(left, right, D, 10, 120).view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h,D", [(10, 30, 64), (10, 31, 64), (10, 31, 65), (8, 640, 70), (8, 641, 70), (8, 641, 16)])
+def test_either_side_of_the_shape_rule(w, h, D):
+    from lux_b200 import api
+    left, right = _images(w, h, w + h)
+    for lr in (True, False):
+        want = C.census_sgm(left, right, D, 10, 120, lr_check=lr)
+        assert np.array_equal(api.CensusStereo.compute(left, right, D, 10, 120, lr_check=lr).view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.gpu
+def test_pairs_of_both_kinds_in_one_batch():
+    """A tall image: pairs of up to 64 disparities walk scanlines, wider ones the lines, in the same batch."""
+    from lux_b200 import api
+    w, h, ds = 20, 100, [32, 100, 60, 200]
+    pairs = [_images(w, h, 5 + k) for k in range(len(ds))]
+    ref = pairs[0][0]
+    others = [p[1] for p in pairs]
+    _, disps = api.CensusStereo.capture(ref, others, ds, [1000.0] * len(ds))
+    for k, d in enumerate(ds):
+        assert np.array_equal(disps[k].view(np.uint32), C.census_sgm(ref, others[k], d, 10, 120).view(np.uint32)), k
