@@ -688,6 +688,7 @@ struct UnitPlane {
   int pad[2];
 };
 
+int cost_unit_tiles(int W, int H) { return ((W + kUnitRun - 1) / kUnitRun) * ((H + kUnitRows - 1) / kUnitRows); }
 size_t cost_unit_phase_bytes(int w, int h, int n_planes) {
   return (size_t)16 * h * unit_pitch(w) + (size_t)n_planes * sizeof(UnitPlane);
 }
@@ -1067,8 +1068,7 @@ int launch_cost(const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t
       uint8_t* ph = reinterpret_cast<uint8_t*>(const_cast<uint32_t*>(a.phase[0]));
       k_unit_planes<<<g.n_planes, 256, 0, s>>>(a, g, zt, reinterpret_cast<UnitPlane*>(ph + (size_t)16 * a.oh[0] * unit_pitch(a.ow[0])));
       count_launches(1);
-      const int tiles_u = ((g.W + kUnitRun - 1) / kUnitRun) * ((g.H + kUnitRows - 1) / kUnitRows);
-      k_cost_unit<<<tiles_u, 32, 0, s>>>(a, g, zt, raw, err);
+      k_cost_unit<<<cost_unit_tiles(g.W, g.H), 32, 0, s>>>(a, g, zt, raw, err);
       kind = 3;
     } else if (a.vcols) {
       const int vruns = ((g.W + kAxRun - 1) / kAxRun) * g.H;

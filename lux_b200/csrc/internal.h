@@ -149,6 +149,7 @@ bool cost_small_wide_layer(int W, int H, int n_planes);
 uint32_t cost_unit_norm(float norm);
 // Bytes of the byte phase images of a w x h camera (and the plane table behind them), for CostArgs::unit.
 size_t cost_unit_phase_bytes(int w, int h, int n_planes);
+int cost_unit_tiles(int W, int H);  // the warps of its launch
 int launch_cost(const CostArgs& a, const LayerGeom& g, const float4* zt, uint8_t* raw, int* err, cudaStream_t s);
 
 // sgm_emulate.cu: the exact replay of the reference's sheared-tile traversal on its line-buffer layout (any layer)

@@ -398,8 +398,10 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
   // an axis-aligned grey pair at scale 1 with the fast layout: the cost kernel that shares block columns between pixels
   ca.vcols = ca.axis && ca.scale == 1 && cost_all_grey(ca) && uniform && L->n % 8 == 0 && !cost_small_wide_layer(W, H, L->n) ? 1 : 0;
   // Cameras of one focal length: every target column lies the same (half-pixel) shift from its pixel. Below 16 M planes and
-  // pixels the plane table and the larger phase images cost more than they save (520x390 D=32: 46 against 37 us).
-  if (ca.vcols && L->volume >= (16u << 20) && cost_unit_phase_bytes(iw[1], ih[1], L->n) < (1ull << 31)) {
+  // pixels the plane table and the larger phase images cost more than they save (520x390 D=32: 46 against 37 us), and below
+  // eight tiles an SM its single warps are too few (us, bytes / triples: 520x390 D=256, 975 tiles, 202 / 168; 640x480 D=256, 1440,
+  // 217 / 266; 2400x120 D=64, 1200, 72 / 71).
+  if (ca.vcols && L->volume >= (16u << 20) && cost_unit_tiles(W, H) >= 1184 && cost_unit_phase_bytes(iw[1], ih[1], L->n) < (1ull << 31)) {
     const float* Wm = ca.warp[0];
     ca.norm_mul = cost_unit_norm(ca.norm);
     ca.unit = Wm[0] == Wm[10] && Wm[5] == Wm[10] && Wm[14] == 0.0f && Wm[10] != 0.0f && ca.norm_mul ? 1 : 0;

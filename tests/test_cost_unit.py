@@ -45,3 +45,12 @@ def test_unit_cost_bit_exact(ctx, oracle, w, h, d, dcx, dcy, density, skip):
         assert np.array_equal(gl.Depth.view(np.uint32), ol["Depth"].view(np.uint32))
     finally:
         gl.close()
+
+
+# its other size rule, 1184 tiles of 120 pixels and two rows: the smallest layers on either side of it, whole and quarter shifts
+# with skipped pixels in layers past it
+@pytest.mark.parametrize("w,h,d,dcx,dcy,density,skip", [
+    (960, 296, 64, 0.0, 0.0, 1.0, 0), (959, 294, 64, 0.0, 0.0, 1.0, 0), (721, 401, 72, 0.5, 0.0, 1.0, 0), (839, 401, 80, 1.25, 0.0, 1.0, 2),
+    (121, 1200, 128, -0.75, 0.0, 1.0, 0)])
+def test_unit_cost_tile_rule(ctx, oracle, w, h, d, dcx, dcy, density, skip):
+    test_unit_cost_bit_exact(ctx, oracle, w, h, d, dcx, dcy, density, skip)
