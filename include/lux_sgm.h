@@ -114,20 +114,25 @@ int lux_sgm_box_filter3(lux_sgm_ctx* ctx, const lux_img_rgba8* src, uint8_t* dst
 #define LUX_LAYER_KEEP_AGG 2     /* keep the final aggregates (DenseLayer.Agg); the depth never needs them */
 #define LUX_LAYER_PREFILTER 4    /* images are unfiltered: apply DenseStereo.BoxFilter3 on the device first */
 #define LUX_LAYER_FORCE_REPLAY 8 /* aggregate with the exact traversal replay even where the fast uniform kernel applies */
-/* The fast uniform aggregation has three forms with the same results: the four paths fused in one wavefront (faster on
- * small layers), the same in a lean form, and the path groups {0,1} / {2,3} as row and column chains (faster from about
- * 2 MP). It takes uniform layers of up to 768 planes; past 256 planes (the L16 pyramid's first layer has 552) only the
- * fused form runs them, whatever these flags ask. By default the library picks by timing (below); these flags force
- * one form (tuning and tests). */
+/* A uniform layer of up to 256 planes and eight columns or more, and most ragged ones, are aggregated by single lines
+ * (sgm_kernel 4), which is the fastest form and waits on nothing; its states need device memory, and where the context's
+ * budget or the device does not have it the solve runs without them. The lines never hold pass +1's aggregates by
+ * themselves, so a uniform layer that keeps them (LUX_LAYER_KEEP_PASS1) takes one of three other forms with the same
+ * results: the four paths fused in one wavefront (faster on small layers), the same in a lean form, and the path groups
+ * {0,1} / {2,3} as row and column chains (faster from about 2 MP). Past 256 planes (to 768; the L16 pyramid's first layer
+ * has 552) the lines' other form runs, and the fused wavefront where it may not. These flags force one of the three,
+ * past 256 planes always the fused one (tuning and tests). */
 #define LUX_LAYER_SGM_FUSED 16
 #define LUX_LAYER_SGM_SPLIT 32
 #define LUX_LAYER_SGM_WAVE 64    /* the fused wavefront in its lean form (progress counters, packed minima) */
-/* Autotuning of the fast form (no counterpart in the reference, which has one CPU loop): with none of the three flags
- * above, a uniform layer of a shape (w, h, planes, tile) not seen before is aggregated once with every fast form on its
- * own cost volume, timed with CUDA events; the fastest is kept for later solves of that shape by every context of the
+/* Autotuning of the three (no counterpart in the reference, which has one CPU loop). It runs only where the lines do not:
+ * with none of the three flags above, the first solve of a shape (w, h, planes, tile) aggregates its own cost volume once
+ * with every form, timed with CUDA events; the fastest is kept for later such solves of that shape by every context of the
  * process (all forms give the same bits, so the result does not depend on the choice). Without autotuning, or for a
- * shape not yet tuned, the choice is by size. lux_sgm_set_tuned_form sets or (form 0) clears a choice, e.g. to restore
- * choices saved from an earlier process. */
+ * shape not yet tuned, the choice is by size. lux_sgm_tuned_form returns the choice, 0 for none: also after solves by
+ * lines, which time nothing. lux_sgm_set_tuned_form sets (1 to 3) or, with form 0, clears a choice. A choice set this way
+ * is followed in place of the lines too, so restoring choices saved from an earlier process gives up the lines for
+ * those shapes; form 4 is no choice to set: it is what runs where none is. */
 int lux_sgm_set_autotune(lux_sgm_ctx* ctx, int32_t on);
 int32_t lux_sgm_tuned_form(int32_t w, int32_t h, int32_t n_planes, int32_t tile);
 int lux_sgm_set_tuned_form(int32_t w, int32_t h, int32_t n_planes, int32_t tile, int32_t form);
@@ -136,7 +141,8 @@ int lux_sgm_set_tuned_form(int32_t w, int32_t h, int32_t n_planes, int32_t tile,
  * images: n_cams camera images (camera 0 = reference), box-FILTERED already unless LUX_LAYER_PREFILTER (as
  * DenseStereoPyramid.Run filters them, DenseStereoSgm.cs:335); gray[k] selects the grey cost weights; prev = the
  * previous layer (NULL for a first layer: every pixel searches all planes). The layer object owns its device state
- * until lux_layer_destroy. LUX_ERR_UNSUPPORTED where the exact replay would need a line buffer (2·(w+2)·(4·MaxHi+5)
+ * until lux_layer_destroy. LUX_ERR_UNSUPPORTED where the exact replay (for a ragged layer, whichever form would run) would
+ * need a line buffer (2·(w+2)·(4·MaxHi+5)
  * u16) past 2^31 - 2^16 elements, which it indexes with 32-bit integers (w beyond about 65,000 pixels). */
 int lux_sgm_layer(lux_sgm_ctx* ctx, int32_t n_cams, const lux_img_rgba8* images, const uint8_t* gray, const lux_calib* calibs,
                   float near_, float far_, const lux_stereo_params* params, int32_t index, int32_t align, const lux_layer* prev,
@@ -163,7 +169,9 @@ typedef struct {
   int32_t sgm_kernel;    /* 0 = the exact traversal replay, 1 = fast, four paths fused, 2 = fast, path groups as chains,
                             3 = fast, four paths fused, lean wavefront, 4 = fast, every path along its own lines */
   int32_t cost_kernel;   /* 0 = per-pixel warps (any layer), 1 = per-row warps (uniform layer), 2 = per-row warps of an axis-aligned
-                            pair, 3 = the same with block columns shared between neighbouring pixels (grey, scale 1) */
+                            pair, 3 = the same on shared data (grey, scale 1): block columns shared between neighbouring pixels, or,
+                            for cameras of one focal length in layers of 16 M planes and pixels and 1184 tiles of 120x2 pixels
+                            or more, four pixels a word */
   int32_t tuned;         /* the fast form the autotuner chose on this solve (it timed every form), 0 when it did not run */
 } lux_layer_info;
 int lux_layer_get_info(const lux_layer* layer, lux_layer_info* info);
@@ -316,9 +324,9 @@ int lux_depth_cache_fetch(lux_sgm_ctx* ctx, const float* cache, int32_t cw, int3
  * implied; prev = NULL, align 8), its depth map copied into out_depth (host, the layer's w*h floats, out_bytes long;
  * NULL: nothing copied). The server copies the request's small arrays at submit; the caller keeps the image data and
  * out_depth alive until lux_server_wait has returned for the ticket. Every result equals the same request solved alone.
- * The workers pick the aggregation form by size (path-group chains from about 2 MP, the fused wavefront below) unless
- * the request's flags name one: the autotuner's choices are timed on an idle GPU and need not be the best beside other
- * requests; the workers do not autotune either. */
+ * A request whose flags name no aggregation form takes what lux_sgm_layer takes (the lines). One that keeps pass +1's
+ * aggregates takes its form by size (path-group chains from about 2 MP, the fused wavefront below): the autotuner's
+ * choices are timed on an idle GPU and need not be the best beside other requests, and the workers do not autotune. */
 typedef struct lux_server lux_server;
 typedef struct {
   int32_t n_cams;

@@ -146,7 +146,8 @@ class Context:
         self.check(self.lib.lux_sgm_set_wait_limit(self.handle, int(ns)))
 
     def set_autotune(self, on: bool):
-        """Untuned uniform layer shapes time every fast aggregation form on their first solve (the default) or not."""
+        """Untuned uniform layer shapes that keep pass +1's aggregates (which the lines never hold) time the three forms that do on
+        their first solve (the default) or not."""
         self.check(self.lib.lux_sgm_set_autotune(self.handle, 1 if on else 0))
 
     def debug_stall(self, block: int):
@@ -268,8 +269,9 @@ class DenseLayer:
         """DenseLayer.Init + Compute (DenseStereoSgm.cs:34-62, 181-232). images: RGBA8 (camera 0 = reference), box-filtered
         already unless prefilter=True (then BoxFilter3 runs on the GPU first, as DenseStereoPyramid.Run does).
         keep_pass1 / keep_agg keep DenseLayer.AggPass1 / Agg readable (the depth needs neither); force_replay aggregates
-        with the exact traversal replay kernel even where the fast uniform kernel applies; sgm picks the form of the fast
-        kernel ("fused" four-path wavefront, "split" path-group chains, "auto" by size)."""
+        with the exact traversal replay kernel even where a fast form applies; sgm forces a form of a uniform layer
+        ("fused" four-path wavefront, "wave" the same in a lean form, "split" path-group chains); "auto": by single lines,
+        or, where pass +1's aggregates are kept, the form the autotuner or the layer's size chooses."""
         ctx = ctx or default_context()
         arr = (L.Img * len(images))()
         keep = []
@@ -752,12 +754,13 @@ SGM_FORM_NAMES = {1: "fused", 2: "split", 3: "wave", 4: "lines"}
 
 
 def tuned_form(w, h, n_planes, tile) -> int:
-    """The fast aggregation form the autotuner chose for a layer shape (1 fused, 2 split, 3 wave), 0 if none yet."""
+    """The form chosen for a layer shape by the autotuner or set_tuned_form (1 fused, 2 split, 3 wave), 0 if none: also after
+    solves by lines, which time nothing."""
     return int(L.load().lux_sgm_tuned_form(w, h, n_planes, tile))
 
 
 def set_tuned_form(w, h, n_planes, tile, form: int):
-    """Sets (1-3) or clears (0) the autotuner's choice for a layer shape."""
+    """Sets (1-3) or clears (0) the choice for a layer shape. A choice set here is followed in place of the lines too."""
     rc = L.load().lux_sgm_set_tuned_form(w, h, n_planes, tile, int(form))
     if rc:
         _raise(rc, "lux_sgm_set_tuned_form failed")

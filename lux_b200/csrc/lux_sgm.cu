@@ -35,7 +35,7 @@ struct lux_sgm_ctx {
   uint64_t wait_limit_ns = kTimeoutNs;  // bound of every device-side wait of the aggregation kernels
   int stall_block = -1;                 // failure-path tests: the block whose cross-block wait can never be satisfied
   int* d_never = nullptr;               // the zero counter that block waits on (nothing writes it)
-  bool autotune = true;                 // untuned layer shapes time every fast form on their first solve
+  bool autotune = true;                 // untuned shapes that the lines do not take time the other fast forms on their first solve
 };
 
 struct DevBuf {
@@ -450,7 +450,7 @@ int build_layer(lux_sgm_ctx* ctx, int n_cams, const uint8_t* const* dimg, const 
     bool tune = false, keep_states = false;
     if (!forced) {
       const TunedForm t = tuned_form(W, H, L->n, p.tile);
-      // The lines form is faster than the other three at every size (4160x3120 D=256: 15.4 against 17.6 ms; 1040x780
+      // The lines form is faster than the other three at every size (4160x3120 D=256: 14.9 against 17.6 ms; 1040x780
       // D=64: 0.64 against 4.5 ms; 520x390 D=32: 0.26 against 2.4 ms) but never holds pass +1's aggregates alone and waits on nothing (debug_stall).
       if (!(flags & LUX_LAYER_KEEP_PASS1) && !t.set_by_caller && ctx->stall_block < 0 && lines_supported(W, L->n)) {
         keep_states = lines_keep_states(W, H, L->n);

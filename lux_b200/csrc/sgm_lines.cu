@@ -16,8 +16,8 @@
 // up to a power of two), so a warp carries 32 / GL neighbouring lines. Two variants, chosen by size (small_form):
 //   * small layers: the four paths of a pass in one launch, each adding its L into the aggregates by reductions in L2 (four
 //     u16 sums in a 64-bit add, none of which can carry). A pass is as long as one line: latency is what such a layer costs.
-//   * large layers, path by path: k_lines_ckpt walks the lines forward and keeps the path's state every kSeg pixels;
-//     k_lines_pair walks them back in segments of kSeg pixels: it makes the forward L of the segment again from the kept
+//   * large layers, path by path: ckpt_lines walks the lines forward and keeps the path's state every kSeg pixels;
+//     pair_lines walks them back in segments of kSeg pixels: it makes the forward L of the segment again from the kept
 //     state, adds it in shared memory to the aggregates staged there, then runs the backward recurrence of the other
 //     pass over the segment. Forward and backward so share one read and one write of the aggregates: per plane and
 //     pixel 22 bytes a layer instead of 36 for eight separate read-modify-write walks, for half as much arithmetic again.
@@ -546,7 +546,7 @@ LUX_DEV void ckpt_lines(const LineArgs& a, int wi, uint2* ring, uint16_t* ckpt, 
 // aggregates (the first path of the layer), 1 adds to them, 2 reads them, takes the winner-take-all and stores them only
 // when they are kept. Per lane and pixel of a segment: 16 bytes of sums and 8 of raw costs in shared memory, refilled by
 // cp.async for the next segment as soon as the backward walk is through with a pixel. Path 2 leaves columns 0 and W-1 to
-// their own chains. Bound by HBM (5.6 TB/s for path 1 of 4160x3120 D=256).
+// their own chains. Bound by HBM (5.6 TB/s for path 1 of 4160x3120 D=256; at 2080x1560 4.5, with issue at 57 %).
 template <int GL, int P, int MODE>
 LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, const uint16_t* ckpt, const uint16_t* ckpt_min) {
   constexpr int LPW = 32 / GL;
@@ -599,7 +599,8 @@ LUX_DEV void pair_lines(const LineArgs& a, int wi, uint4* sum, uint2* rawp, cons
   for (int seg = nseg - 1; seg >= 0; seg--) {
     const int t0 = seg * kSeg;
     cp_async_wait<0>();
-    // a whole segment clear of the sides (a new line; column 1, where pass -1's states are kept)
+    // a whole segment clear of the sides (a new line; column 1, where pass -1's states are kept). Where two lines of a warp end
+    // a step apart, one of them is at a side in the segment in which the shorter one ends, whose walk back then starts below.
     bool odd = t0 + kSeg > NS;
     if (P == 1) odd |= x0 <= 1 || x0 + kSeg >= W;
     if (P == 3) odd |= x0 == W - 1 || x0 < kSeg;
