@@ -41,11 +41,19 @@ W_, H_, D_, TILE, BITS, DESC = WORKLOADS["pair13mp"]
 # Algorithmic HBM bytes per disparity element (DE = one pixel x one plane) of a layer's aggregation, aggregates not kept:
 # pass +1 reads the u8 raw volume (1) and writes the u16 aggregates (2); pass -1 reads both again (1 + 2).
 BYTES_PER_DE_AGG = 6
-# DRAM bytes (read + write) per DE of a layer's aggregation as built (the path-group chains: 4 launches per layer),
-# from ncu dram__bytes_read.sum + dram__bytes_write.sum of the four k_chains launches of the 2080x1560 D=256 pair:
-# 2.655 + 4.315 + 4.317 + 2.730 GB = 14.02 GB for 830.7 MDE. The split design trades these extra bytes (aggregates read
-# and written by both path groups, raw costs read by each) for a critical path of W or H steps.
-TRAFFIC_PER_DE_LAYER = 14.02e9 / (2080 * 1560 * 256)
+# DRAM bytes (read + write) per DE of a layer's aggregation as built, from ncu dram__bytes_read.sum + dram__bytes_write.sum at
+# 2080x1560 D=256 (830.7 MDE), per form: the lines with kept states 18.27 GB (five walks; the aggregates read and written once a
+# path, the raw costs read twice), the path-group chains 14.02 GB (four launches).
+TRAFFIC_GB_3MP = {4: 18.27, 2: 14.02}
+FORM_KERNELS = {0: "k_sgm_emulate", 1: "k_sgm_uniform", 2: "k_chains", 3: "k_wave", 4: "k_lines_walk / k_lines_pass"}
+
+
+def traffic_per_de(form):
+    """DRAM bytes per DE of the form that ran, None where it was not measured (the lines below their size rule keep no states)."""
+    planes = D_ or 160  # (a capture's layer: 160 planes and more)
+    if form not in TRAFFIC_GB_3MP or (form == 4 and (planes <= 32 or W_ * H_ * planes < (480 if planes <= 128 else 240) << 20)):
+        return None
+    return TRAFFIC_GB_3MP[form] * 1e9 / (2080 * 1560 * 256)
 
 
 def metric():
@@ -62,8 +70,7 @@ def args_():
     p.add_argument("--impl", default="lux", choices=["lux", "reference"])
     p.add_argument("--no-cpu-baseline", action="store_true")
     p.add_argument("--sgm", default="auto", choices=["auto", "split", "wave", "fused"],
-                   help="aggregation form of the timed solves (auto: the autotuner's choice, timed on the first solve of the "
-                        "shape; a fixed form for profiler runs, whose timings would mislead the tuner)")
+                   help="aggregation form of the timed solves (auto: the library's choice, the lines wherever they apply)")
     p.add_argument("--no-served", action="store_true",
                    help="leave out the served stream and the batched capture objects of the default line")
     p.add_argument("--serve", action="store_true",
@@ -72,7 +79,7 @@ def args_():
     p.add_argument("--requests", type=int, default=400)
     p.add_argument("--rate", type=float, default=40.0,
                    help="mean arrivals per second of the served stream (40/s: below what one request at a time keeps up "
-                        "with, about 53/s, so the latencies compare the serving forms, not a growing backlog)")
+                        "with, about 93/s, so the latencies compare the serving forms, not a growing backlog)")
     p.add_argument("--slots", type=int, default=2,
                    help="worker contexts of the request server (2 measured best: 3 stretches large requests' tails)")
     p.add_argument("--sweep", action="store_true",
@@ -300,6 +307,8 @@ def run_lux(a):
     pk = peaks()
     # per layer: the algorithmic bytes of both passes over the device time of the layer's aggregation launches
     achieved = BYTES_PER_DE_AGG * de / (sgm_ms / 1e3) / 1e9
+    form = inf_v[0][3] if inf_v else -1
+    per_de = traffic_per_de(form)
     out = {
         "metric": metric(), "value": value, "unit": "MDE/s", "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
         "ms_per_step": ms_v / a.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -307,13 +316,12 @@ def run_lux(a):
         "config": {"workload": DESC,
                    "parallelism": f"replicas x{world}", "l2": l2_note(),
                    "stages_ms": {"cost": cost_ms, "sgm_2_passes": sgm_ms, "wta": wta_ms},
-                   "sgm_kernel": {0: "exact-replay", 1: "fused-wavefront", 2: "path-group-chains", 3: "lean-wavefront", 4: "lines"}.get(
-                       inf_v[0][3] if inf_v else -1)},
+                   "sgm_kernel": {0: "exact-replay", 1: "fused-wavefront", 2: "path-group-chains", 3: "lean-wavefront", 4: "lines"}.get(form)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk.get("hbm_gbs"), "unit": "GB/s",
-                     "frac": achieved / pk.get("hbm_gbs"), "traffic": TRAFFIC_PER_DE_LAYER * de,
-                     "kernel": "SGM aggregation of one layer (both passes; 4 chain launches, or 2 fused ones below 2 MP)",
-                     "bytes_per_de": BYTES_PER_DE_AGG, "traffic_per_de": TRAFFIC_PER_DE_LAYER,
-                     "traffic_source": "ncu dram__bytes_read+write of the four 2080x1560 D=256 k_chains launches, scaled by DE",
+                     "frac": achieved / pk.get("hbm_gbs"), "traffic": per_de * de if per_de else None,
+                     "kernel": f"SGM aggregation of one layer (both passes): {FORM_KERNELS.get(form, form)}",
+                     "bytes_per_de": BYTES_PER_DE_AGG, "traffic_per_de": per_de,
+                     "traffic_source": "ncu dram__bytes_read+write of the same form at 2080x1560 D=256, scaled by DE" if per_de else None,
                      "peak_source": "fallback" if pk.get("fallback") else "MEASURED_PEAKS.json hbm_gbs (measured)"},
         "e2e": {"value": e2e, "unit": "MDE/s", "h2d_bytes_per_step": h2d_bytes, "d2h_bytes_per_step": W_ * H_ * 4,
                 "path": ("host uint16 12-bit samples -> lux_image_from_grey16 -> lux_sgm_layer -> depth read back"
@@ -391,9 +399,11 @@ def serve_stream(a):
 
     # warm-up: every input solved once (builds, pools, lazy module loading)
     ctx = api.Context(0)
+    forms = {}  # of plain solves; a request that names no form takes the same
     for kind in pool:
         for r in pool[kind]:
             L = api.DenseLayer.compute(r[0], *r[1:6], prefilter=True, ctx=ctx)
+            forms[kind] = api.SGM_FORM_NAMES.get(L.sgm_kernel, "replay")
             L.close()
 
     def plain():
@@ -449,10 +459,6 @@ def serve_stream(a):
         return {"req_per_s": len(picks) / tot, "p50_ms": float(np.percentile(lat, 50) * 1e3),
                 "p99_ms": float(np.percentile(lat, 99) * 1e3), "mde_per_s": de / tot / 1e6, "wall_s": tot}
 
-    shapes = {"preview": (520, 390, 32), "pair13mp": (4160, 3120, 128), "capture10": (2080, 1560, n_mc)}
-    # plain: the library's default (the autotuner's choice); served: the server's choice by size
-    forms = {k: {"plain": api.SGM_FORM_NAMES.get(api.tuned_form(w, h, n, 64), "size rule"),
-                 "served": "split" if w * h >= 2000000 else "fused"} for k, (w, h, n) in shapes.items()}
     return {"workload": f"{a.requests} Poisson arrivals at {a.rate}/s: {mix}", "slots": a.slots, "hbm_budget_gb": 120,
             "sgm_forms": forms, "served": stats(lat_s, tot_s), "plain": stats(lat_p, tot_p)}
 
@@ -493,18 +499,19 @@ def capture_batched_vs_plain(a, steps=5, warmup=3):
         return e0.elapsed_time(e1) / steps
 
     ms_b, ms_p = timed(batched), timed(plain)
-    # the size rule the autotuner replaces (path-group chains from about 2 MP, so every layer here): the same work
+    # the same work by the path-group chains
     ms_bf, ms_pf = timed(lambda: batched("split")), timed(lambda: plain("split"))
-    form = api.SGM_FORM_NAMES.get(api.tuned_form(2080, 1560, n, mc.params.tile), "untuned")
+    L = api.DenseLayer.compute(dev_imgs, mc.gray, mc.calibs, mc.near, mc.far, mc.params, prefilter=True, ctx=ctx)
+    form = api.SGM_FORM_NAMES.get(L.sgm_kernel, "replay")
+    L.close()
     ctx.close()
     return {"workload": "2080x1560 reference + 10 module cameras (1-6 MP crops, focal 1.0-2.7x, D_k 64-192), u8",
             "batched": {"ms_per_capture": ms_b, "planes": n, "mde_per_s": 2080 * 1560 * n / ms_b / 1e3, "sgm": form,
                         "note": "one layer summing the ten cameras' costs (the reference's multi-view sum)"},
             "plain": {"ms_per_capture": ms_p, "planes": n_k, "mde_per_s": sum(2080 * 1560 * k for k in n_k) / ms_p / 1e3,
                       "note": "ten two-camera layers one after another"},
-            "size_rule": {"batched_ms": ms_bf, "plain_ms": ms_pf,
-                          "note": "the same two jobs with the aggregation form fixed by size (path-group chains), "
-                                  "against the autotuned forms above"}}
+            "chains": {"batched_ms": ms_bf, "plain_ms": ms_pf,
+                       "note": "the same two jobs with the aggregation by path-group chains"}}
 
 
 def run_serve(a):
@@ -781,9 +788,9 @@ def run_stereo(a):
 
 def run_census(a):
     """The opt-in census stereo mode on the workload's pair (default: 4160x3120, D=256): value = W·H·D per second with the
-    images in HBM and the disparities left there; e2e from host images to host disparities. Roofline (HBM), the
-    aggregation's algorithmic bytes: the eight path launches each read the u8 cost volume once and read-modify-write the
-    u16 path sums (the first only writes): 8·1 + 7·4 + 2 = 38 bytes per DE."""
+    images in HBM and the disparities left there; e2e from host images to host disparities. Roofline (HBM): the u8 cost
+    volume written once and, like a layer's aggregation, read twice, the u16 sums written twice and read once, 7 + 2 (the
+    right image's winners) = 9 bytes per DE; traffic as built, from ncu at 2080x1560 D=128 (10.9 GB for 415.3 MDE)."""
     import torch
     from lux_b200 import _lib, api
     if int(os.environ.get("RANK", "0")) != 0:
@@ -842,13 +849,13 @@ def run_census(a):
     ms_e, _ = timed(lambda: step(False), a.steps)
     de = W_ * H_ * D
     pk = peaks()
-    achieved = 38 * de / (ms_v / 1e3) / 1e9  # the whole step's time: an upper bound on the aggregation's
+    achieved = 9 * de / (ms_v / 1e3) / 1e9  # over the whole step's time
     out = {"metric": f"census SGM MDE/s (W·H·D per second), {W_}x{H_} pair D={D}, opt-in mode", "value": de / (ms_v / 1e3) / 1e6,
            "unit": "MDE/s", "n_gpus": 1, "steps": a.steps, "warmup": a.warmup, "ms_per_step": ms_v, "higher_is_better": True,
            "scaling": "weak", "vs_baseline": None, "dtype": "u8 cost / u16 aggregation", "data": "synthetic",
            "config": {"workload": DESC + " (census mode: 9x7 census, P1 10, P2 120, subpixel, left/right)", "l2": l2_note()},
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk.get("hbm_gbs"), "unit": "GB/s", "frac": achieved / pk.get("hbm_gbs"),
-                        "traffic": None, "kernel": "the whole census step (38 B/DE of aggregation over the step's time)",
+                        "traffic": 10.9e9 / (2080 * 1560 * 128) * de, "kernel": "the whole census step (9 B/DE over the step's time)",
                         "peak_source": "fallback" if pk.get("fallback") else "MEASURED_PEAKS.json hbm_gbs (measured)"},
            "e2e": {"value": de / (ms_e / 1e3) / 1e6, "unit": "MDE/s", "h2d_bytes_per_step": 2 * W_ * H_ * 4, "d2h_bytes_per_step": W_ * H_ * 4},
            "gpu_launches": int(launches), "clocks": clk.summary()}
@@ -979,7 +986,7 @@ def pyramid_job(a, w, h, steps, warmup, cpu=True):
            "captures_per_s": 1e3 / ms, "mde_per_s": de / (ms / 1e3) / 1e6, "gpu_launches": int(launches),
            "clocks": clk.summary(),
            "upsample": {"ms": ms_up, "gb_per_s": up_bytes / ms_up / 1e6, "frac": up_bytes / ms_up / 1e6 / peak,
-                        "bytes": up_bytes, "note": "k_shift_resize + k_bilateral, of the measured HBM copy bandwidth"},
+                        "bytes": up_bytes, "note": "k_shift_resize + k_bilateral_quads, of the measured HBM copy bandwidth"},
            "layers": [{"w": W, "h": H, "planes": n, "mean_cap": round(mc, 1), "sgm_kernel": sk, "cost_kernel": ck,
                        "ms_cost": round(c, 3), "ms_sgm": round(g, 3), "ms_wta": round(t, 3)}
                       for (W, H, n, sk, ck, c, g, t, mc) in info]}
